@@ -70,7 +70,6 @@ def draw(rng):
                        "learned", "train"])
     c = dict(path=path)
 
-
     def tet(lo, hi):
         n = _log_int(rng, lo, hi)
         nx, ny, nz = (min(hi, max(lo, round(n * rng.uniform(0.75, 1.33)))) for _ in range(3))
