@@ -30,7 +30,7 @@ def pytest_configure(config):
         b.build()
     ref_lib = ROOT / "oracle" / "_ref" / "libcfdx_ref.so"
     demo = ROOT / "oracle" / "_ref" / "cfdx_adapter_demo"
-    if (not ref_lib.exists() or not demo.exists()) and REF_SRC.exists():
+    if (not ref_lib.exists() or not demo.exists()) and (REF_SRC / "src").is_dir():
         subprocess.run(["make", "-s", "-C", str(ROOT / "oracle"), "ref", "oracle", "adapter", f"REF_ROOT={REF_SRC}"],
                        check=True)
     c_lib = ROOT / "oracle" / "_build" / "libcfdx_oracle.so"
