@@ -70,6 +70,27 @@ def test_composed_training_gradient_matches_oracle(bound, oracle):
     assert np.linalg.norm(grad - grad_ref) <= 1e-4 * np.linalg.norm(grad_ref)
 
 
+@pytest.mark.parametrize("n,batch", [(1, 3), (1, 70), (2, 5), (3, 8), (5, 1)])
+def test_training_gradient_tiles_and_pair_chunks(ctx, n, batch):
+    """Pairs of fewer cells than a 64-cell tile (tiles that hold several pairs),
+    batches beyond the 64 pairs taken together, remainder tiles."""
+    m = cases.simple_mesh(n)
+    mesh = cg.Mesh(ctx, m)
+    g = mesh.geometry()
+    U, rAU, aP, p, fixed, value = cases.simple_fields(m, g["cell_centres"])
+    A, b, phi, grad = cg.assemble_pressure_correction(mesh, U, rAU, p, 1.0, fixed, value)
+    G = mo.Graph(*A.to_csr(), g["cell_volumes"], aP)
+    net = cg.LearnedPreconditioner(ctx, seed=3)
+    net.bind(mesh, A, aP)
+    net.set_parameters(mo.init_params(5).astype(np.float32))
+    R, E = _pairs(G, batch, seed=n)
+    loss, grad = net.loss_grad(R, E)
+    loss_ref, grad_ref = mo.loss_and_grad(net.parameters().astype(np.float64), G, list(zip(R, E)))
+    # as above: FP32 kernels against the FP64 oracle
+    assert abs(loss - loss_ref) <= 1e-5 * abs(loss_ref)
+    assert np.linalg.norm(grad - grad_ref) <= 1e-4 * np.linalg.norm(grad_ref)
+
+
 def test_tensor_core_inference_matches_oracle(bound):
     G, net, theta = bound["G"], bound["net"], bound["theta"]
     r = np.random.default_rng(4).standard_normal(G.n)
