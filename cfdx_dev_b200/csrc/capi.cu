@@ -65,11 +65,14 @@ __global__ void k_scale(int n, const double* a, const double* b, double* out) {
 // max |a_k| over the stored values (diagnose_matrix max_abs_value); a
 // non-finite value makes the slot NaN.
 __global__ void k_absmax_values(int64_t nnz, const double* va, unsigned long long* bits) {
+    __shared__ double sm[32];
     double m = 0.0;
     for (int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; k < nnz; k += int64_t(gridDim.x) * blockDim.x)
         m = fmax(m, fabs(va[k]));
-    // non-negative doubles order like their bit patterns
-    atomicMax(bits, static_cast<unsigned long long>(__double_as_longlong(m)));
+    // non-negative doubles order like their bit patterns; one atomic per block
+    // (one per thread took 145 us on 222,208 values)
+    m = block_max(m, sm);
+    if (threadIdx.x == 0) atomicMax(bits, static_cast<unsigned long long>(__double_as_longlong(m)));
 }
 
 // measure_matrix_characteristics (core/linalg/matrix_diagnostics.h:317-355):
@@ -688,8 +691,8 @@ KrylovResult run_krylov(cfdxg_context* ctx, const cfdxg_matrix* A, cfdxg_amg* am
                 check_launch(ctx);
                 return true;
             };
-        return cg_solve(ctx, A, b, x, max_it, tol, pc, setup, req.preconditioner == CFDXG_PC_OWN_DIAGONAL,
-                        null_space);
+        return cg_solve(ctx, A, b, x, max_it, tol, pc, setup,
+                        req.preconditioner == CFDXG_PC_OWN_DIAGONAL ? inv_diag : nullptr, null_space);
     }
     // Learned stage: dropped for the rest of the solve (plain AMG fallback)
     // as soon as an iteration fails to cut the residual estimate by 10%.

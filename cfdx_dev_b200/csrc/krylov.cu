@@ -832,6 +832,201 @@ __global__ void k_cg_direction(int n, double* __restrict__ p, const double* __re
     if (i < n) p[i] = z[i] + beta * p[i];
 }
 
+// ---- CG with the solver's own diagonal in one persistent kernel
+//
+// On the sizes this solver serves (the Poisson driver's meshes) an iteration
+// is a few microseconds of work; as separate kernels with a read-back of its
+// scalars it took 82 us at 32,768 cells.  Here the whole iteration runs in one
+// cooperative launch (every block resident) with two grid-wide reductions:
+//
+//   1. p = z + beta p (each gathered entry formed where it is read, the own
+//      one stored for step 2), A p and b - A x in one pass over the matrix;
+//      reduce p . A p, and |b - A x| of the previous iteration's x
+//   2. x += alpha p, r -= alpha A p, z = r / d; reduce r . z, r . r and the
+//      finite checks
+//
+// Every block adds the blocks' partials in the same fixed order, so all take
+// the same decisions and the result is deterministic.  The kernel runs on as
+// long as the reference's loop would plainly continue; at anything else
+// (convergence, a residual replacement, a breakdown, the iteration limit, a
+// residual outside the range in which plain squares are exact enough) it stops
+// before x changes again and the host decides on that iteration.
+enum CgRunSlot : int {
+    kRunCode = 20, kRunIterations = 21, kRunPAp = 22, kRunRsOld = 23, kRunRsNew = 24, kRunRR = 25, kRunXBad = 26,
+    kRunZBad = 27, kRunP = 28, kRunCount = 29
+};
+enum CgRunCode : int { kRunDecide = 0, kRunCurvature = 1, kRunStalled = 2 };
+constexpr int kRunThreads = kT;
+constexpr int kRunBlocksPerSm = 3;   // 80 registers; four per SM spilled
+// A barrier gives up after this many polls (about a second): the blocks are
+// co-resident, so only a failure elsewhere on the GPU could keep one away.
+constexpr unsigned kRunSpinLimit = 1u << 20;
+
+// Sums v[0..NS) and takes the maximum of v[NS..NV) over the grid; every thread
+// gets the results.  Also a grid-wide barrier: what the block's threads wrote
+// before it is visible to every block after it.  Returns false when it gave up.
+template <int NS, int NV>
+__device__ __forceinline__ bool grid_combine(double (&v)[NV], double* part, unsigned* counter, unsigned target) {
+    constexpr int kW = kRunThreads / 32;
+    __shared__ double sm[NV][kW];
+    __shared__ double total[NV];
+    __shared__ int gave_up;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+        double t = v[q];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double u = __shfl_xor_sync(0xffffffffu, t, o);
+            t = q < NS ? t + u : fmax(t, u);
+        }
+        if (lane == 0) sm[q][warp] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x < NV) {
+        const int q = threadIdx.x;
+        double t = sm[q][0];
+#pragma unroll
+        for (int w = 1; w < kW; ++w) t = q < NS ? t + sm[q][w] : fmax(t, sm[q][w]);
+        __stcg(part + q * gridDim.x + blockIdx.x, t);
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(counter, 1u);
+        unsigned seen = 0, polls = 0;
+        do {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
+        } while (seen < target && ++polls < kRunSpinLimit);
+        gave_up = seen < target;
+        __threadfence();
+    }
+    __syncthreads();
+    if (gave_up) return false;
+    if (warp < NV) {
+        double t = 0.0;
+        for (int b = lane; b < static_cast<int>(gridDim.x); b += 32) {
+            const double u = __ldcg(part + warp * gridDim.x + b);
+            t = warp < NS ? t + u : fmax(t, u);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double u = __shfl_xor_sync(0xffffffffu, t, o);
+            t = warp < NS ? t + u : fmax(t, u);
+        }
+        if (lane == 0) total[warp] = t;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NV; ++q) v[q] = total[q];
+    return true;
+}
+
+// p0 holds the first search direction, z = r / d and rsold = r . z; the
+// direction of iteration k alternates between p0 and p1.  x, r, z and the
+// directions are written here and read by other blocks: every read of them
+// goes to L2.
+__global__ void __launch_bounds__(kRunThreads, kRunBlocksPerSm) k_cg_run(
+    int n, const int* __restrict__ ro, const int* __restrict__ co, const double* __restrict__ va,
+    const double* __restrict__ b, const double* __restrict__ d, double* x, double* r, double* z, double* p0, double* p1,
+    double* Ap, double rsold, double tol_abs, int limit, double* part, unsigned* counter, double* slots) {
+    const int stride = gridDim.x * kRunThreads;
+    const int first_row = blockIdx.x * kRunThreads + threadIdx.x;
+    double* half[2] = {part, part + 4 * gridDim.x};
+    unsigned arrivals = 0;
+    double beta = 0.0, rsnew = 0.0, rr = 0.0, xbad = 0.0, zbad = 0.0;
+    double* pk = p0;      // the current direction
+    double* pn = p1;      // the next one's buffer
+    int code = kRunDecide;
+    double pAp = 0.0;
+    int it = 1;
+    for (;; ++it) {
+        double s1[3] = {0.0, 0.0, 0.0};
+        for (int i = first_row; i < n; i += stride) {
+            double ap = 0.0, ax = 0.0;
+            const int e = ro[i + 1];
+#pragma unroll 4
+            for (int k = ro[i]; k < e; ++k) {
+                const int c = co[k];
+                const double a = va[k];
+                const double pc = it == 1 ? __ldcg(pk + c) : __ldcg(z + c) + beta * __ldcg(pk + c);
+                ap += a * pc;
+                ax += a * __ldcg(x + c);
+            }
+            double pi = __ldcg(pk + i);
+            if (it > 1) {
+                pi = __ldcg(z + i) + beta * pi;
+                __stcg(pn + i, pi);
+            }
+            __stcg(Ap + i, ap);
+            const double rv = b[i] - ax;
+            s1[0] += pi * ap;
+            s1[1] += rv * rv;
+            s1[2] = fmax(s1[2], fabs(rv));
+        }
+        if (it > 1) {
+            double* t = pk;
+            pk = pn;
+            pn = t;
+        }
+        arrivals += gridDim.x;
+        if (!grid_combine<2, 3>(s1, half[0], counter, arrivals)) {
+            code = kRunStalled;
+            break;
+        }
+        pAp = s1[0];
+        if (it > 1) {
+            // iteration it - 1 is complete: does the loop plainly continue?
+            const double res = sqrt(s1[1]), rn = sqrt(rr);
+            const bool in_range = isfinite(s1[1]) && s1[2] > 1e-140 && s1[2] < 1e140;
+            const bool replace = isfinite(rn) && rn <= tol_abs;
+            if (xbad > 0.0 || zbad > 0.0 || !isfinite(rsnew) || !in_range || res <= tol_abs || replace || it > limit)
+                break;
+            rsold = rsnew;
+        }
+        if (!(pAp > 0.0) || !isfinite(pAp) || !isfinite(rsold / pAp)) {
+            code = kRunCurvature;
+            break;
+        }
+        const double alpha = rsold / pAp;
+        double s2[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int i = first_row; i < n; i += stride) {
+            const double xi = __ldcg(x + i) + alpha * __ldcg(pk + i);
+            const double ri = __ldcg(r + i) - alpha * __ldcg(Ap + i);
+            const double zi = ri / d[i];
+            __stcg(x + i, xi);
+            __stcg(r + i, ri);
+            __stcg(z + i, zi);
+            s2[0] += ri * zi;
+            s2[1] += ri * ri;
+            if (!isfinite(xi) || !isfinite(ri)) s2[2] = 1.0;
+            if (!isfinite(zi)) s2[3] = 1.0;
+        }
+        arrivals += gridDim.x;
+        if (!grid_combine<2, 4>(s2, half[1], counter, arrivals)) {
+            code = kRunStalled;
+            break;
+        }
+        rsnew = s2[0];
+        rr = s2[1];
+        xbad = s2[2];
+        zbad = s2[3];
+        beta = rsnew / rsold;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        slots[kRunCode] = code;
+        slots[kRunIterations] = it - 1;
+        slots[kRunPAp] = pAp;
+        slots[kRunRsOld] = rsold;
+        slots[kRunRsNew] = rsnew;
+        slots[kRunRR] = rr;
+        slots[kRunXBad] = xbad;
+        slots[kRunZBad] = zbad;
+        slots[kRunP] = pk == p0 ? 0.0 : 1.0;   // the buffer of the next iteration's direction
+    }
+}
+
 // flag = 1 when any of a[0..n) is not finite
 __global__ void k_any_nonfinite(int64_t n, const double* __restrict__ a, double* flag) {
     for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
@@ -1338,7 +1533,7 @@ KrylovResult projected_gmres_solve(cfdxg_context* ctx, const cfdxg_matrix* A, co
 // host takes the reference's decisions in the reference's order.
 KrylovResult cg_solve(cfdxg_context* ctx, const cfdxg_matrix* A, const double* b, double* x, int64_t max_iter,
                       double tolerance, const RightPreconditioner& pc, const std::function<bool()>* setup,
-                      bool own_diagonal, bool null_space) {
+                      const double* own_diagonal, bool null_space) {
     KrylovResult result;
     const int64_t n = A->n;
     if (n == 0) return result;   // NOT_APPLICABLE
@@ -1357,7 +1552,11 @@ KrylovResult cg_solve(cfdxg_context* ctx, const cfdxg_matrix* A, const double* b
     auto project = [&](double* v) {
         if (null_space) E.project(v);
     };
-    DevBuf<double> p(n), z(n), Ap(n);
+    // the direction(s), z and A p in the workspace's Krylov basis blocks (at least 2 n, n and n)
+    double* const p = ws.V.get();
+    double* const p_other = ws.V.get() + n;
+    double* const z = ws.Z.get();
+    double* const Ap = ws.w.get();
     double* r = ws.r.get();
     double* rv = ws.tmp.get();
     auto zero_flags = [&]() {
@@ -1371,8 +1570,8 @@ KrylovResult cg_solve(cfdxg_context* ctx, const cfdxg_matrix* A, const double* b
     };
     auto apply = [&]() {
         ++result.preconditioner_applications;
-        if (!pc(r, z.get(), 0)) return false;
-        project(z.get());                                            // :203
+        if (!pc(r, z, 0)) return false;
+        project(z);                                            // :203
         return true;
     };
 
@@ -1431,26 +1630,104 @@ KrylovResult cg_solve(cfdxg_context* ctx, const cfdxg_matrix* A, const double* b
     E.copy(r, rv);
     zero_flags();
     if (!apply()) return failed(CFDXG_NOT_APPLICABLE, 0, initial);
-    dot_check(r, z.get(), kCgRsOld);
-    E.copy(p.get(), z.get());
+    dot_check(r, z, kCgRsOld);
+    E.copy(p, z);
     E.fetch(kCgCount);
     if (E.host(kCgZBad) > 0.0) return failed(CFDXG_NOT_APPLICABLE, 0, initial);
     double rsold = E.host(kCgRsOld);
     if (!std::isfinite(rsold)) return failed(CFDXG_DIVERGED, 0, initial);
     if (!(rsold > 0.0)) return failed(CFDXG_NOT_APPLICABLE, 0, initial);
 
+    // r = b - A x (in rv), z = M^-1 r, p = z and rsold = r . z (fetched)
+    auto restart_from_residual = [&]() {
+        E.copy(r, rv);
+        project(r);
+        zero_flags();
+        if (!apply()) return false;
+        dot_check(r, z, kCgRsOld);
+        E.copy(p, z);
+        E.fetch(kCgCount);
+        return true;
+    };
+
+    if (own_diagonal && !null_space) {
+        // the persistent kernel, relaunched after every decision of the host
+        int64_t done = 0;
+        double* direction[2] = {p, p_other};
+        int current = 0;
+        const int blocks = std::min(blocks_for(n, kRunThreads),
+                                    std::min(kRunBlocksPerSm, resident_per_sm<k_cg_run>()) * ctx->sm_count);
+        while (done < max_iter) {
+            CFDXG_CUDA(cudaMemsetAsync(ctx->scratch.ticket + 4, 0, sizeof(unsigned), ctx->stream));
+            const int limit = static_cast<int>(std::min<int64_t>(max_iter - done, 1 << 30));
+            {
+                ProfScope ps(ctx, "cg_own_diagonal", 0.0);
+                int nn = ni;
+                const int *ro = A->ro.get(), *co = A->co.get();
+                const double* va = A->va.get();
+                double *p0 = direction[current], *p1 = direction[1 - current], *zz = z, *ap = Ap,
+                       *part = ws.mpartial.get(), *slots = E.slot(0);
+                unsigned* counter = ctx->scratch.ticket + 4;
+                void* args[] = {&nn, &ro, &co, &va, &b, &own_diagonal, &x, &r, &zz, &p0, &p1, &ap, &rsold,
+                                const_cast<double*>(&tol_abs), const_cast<int*>(&limit), &part, &counter, &slots};
+                CFDXG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_cg_run), dim3(blocks),
+                                                       dim3(kRunThreads), args, 0, ctx->stream));
+                check_launch(ctx);
+            }
+            E.residual(b, x, rv);
+            E.norm2(rv, kCgRes);
+            E.fetch(kRunCount);
+            const double res = E.host(kCgRes);
+            const int code = static_cast<int>(E.host(kRunCode));
+            const int64_t ran = static_cast<int64_t>(E.host(kRunIterations));
+            if (code == kRunStalled) throw Error(CFDXG_ERR_CUDA, "CG: a grid-wide barrier was not reached in time");
+            done += ran;
+            result.preconditioner_applications += ran;
+            if (code == kRunCurvature) {
+                ++result.preconditioner_applications;
+                const double pAp = E.host(kRunPAp);
+                if (!(pAp > 0.0) || !std::isfinite(pAp)) return failed(CFDXG_NOT_APPLICABLE, done + 1, res);
+                return failed(CFDXG_DIVERGED, done + 1, res);
+            }
+            if (E.host(kRunXBad) > 0.0) return failed(CFDXG_DIVERGED, done, res);
+            if (E.host(kRunZBad) > 0.0) return failed(CFDXG_NOT_APPLICABLE, done, res);
+            const double rsnew = E.host(kRunRsNew);
+            if (!std::isfinite(rsnew)) return failed(CFDXG_DIVERGED, done, res);
+            if (res <= tol_abs) return finish(CFDXG_CONVERGED, done, res);
+            // :321-352 the residual replacement of the solver's own diagonal
+            const double rr = std::sqrt(E.host(kRunRR));
+            if (std::isfinite(rr) && rr <= tol_abs && res > tol_abs) {
+                ++result.residual_replacements;
+                if (result.first_residual_replacement == 0) result.first_residual_replacement = done;
+                result.last_residual_replacement = done;
+                if (!restart_from_residual()) return failed(CFDXG_NOT_APPLICABLE, done, res);
+                const double replaced = E.host(kCgRsOld);
+                if (E.host(kCgZBad) > 0.0) return failed(CFDXG_NOT_APPLICABLE, done, res);
+                if (!std::isfinite(replaced) || !(replaced > 0.0)) return finish(CFDXG_MAX_ITER_REACHED, done, res);
+                rsold = replaced;
+                current = 0;
+            } else {
+                rsold = rsnew;
+                if (E.host(kRunP) > 0.0) current = 1 - current;
+            }
+        }
+        E.residual(b, x, rv);
+        E.norm2(rv, kCgRes);
+        return finish(CFDXG_MAX_ITER_REACHED, max_iter, E.scalar(kCgRes));
+    }
+
     double at_last_replacement = std::numeric_limits<double>::infinity();
     for (int64_t iter = 1; iter <= max_iter; ++iter) {
         zero_flags();
-        E.spmv(p.get(), Ap.get());
-        project(Ap.get());                                           // :262
-        E.dot(p.get(), Ap.get(), kCgPAp);
-        k_cg_update<<<gb, kT, 0, ctx->stream>>>(ni, x, r, p.get(), Ap.get(), E.slot(0));
+        E.spmv(p, Ap);
+        project(Ap);                                           // :262
+        E.dot(p, Ap, kCgPAp);
+        k_cg_update<<<gb, kT, 0, ctx->stream>>>(ni, x, r, p, Ap, E.slot(0));
         check_launch(ctx);
         project(x);                                                  // :295-298
         project(r);
         if (!apply()) return failed(CFDXG_NOT_APPLICABLE, iter, std::numeric_limits<double>::quiet_NaN());
-        dot_check(r, z.get(), kCgRsNew);
+        dot_check(r, z, kCgRsNew);
         E.residual(b, x, rv);
         E.norm2(rv, kCgRes);
         E.dot(r, r, kCgRR2);
@@ -1472,22 +1749,16 @@ KrylovResult cg_solve(cfdxg_context* ctx, const cfdxg_matrix* A, const double* b
                 ++result.residual_replacements;
                 if (result.first_residual_replacement == 0) result.first_residual_replacement = iter;
                 result.last_residual_replacement = iter;
-                E.copy(r, rv);
-                project(r);                                          // :376
-                zero_flags();
-                if (!apply()) return failed(CFDXG_NOT_APPLICABLE, iter, res);
-                dot_check(r, z.get(), kCgRsOld);
-                E.copy(p.get(), z.get());
-                E.fetch(kCgCount);
+                if (!restart_from_residual()) return failed(CFDXG_NOT_APPLICABLE, iter, res);   // :376
                 const double replaced = E.host(kCgRsOld);
                 if (E.host(kCgZBad) > 0.0) return failed(CFDXG_NOT_APPLICABLE, iter, res);
                 if (!std::isfinite(replaced) || !(replaced > 0.0)) return finish(CFDXG_MAX_ITER_REACHED, iter, res);
                 rsold = replaced;
                 continue;
             }
-            k_cg_direction<<<gb, kT, 0, ctx->stream>>>(ni, p.get(), z.get(), E.slot(0));
+            k_cg_direction<<<gb, kT, 0, ctx->stream>>>(ni, p, z, E.slot(0));
             check_launch(ctx);
-            project(p.get());                                        // :558
+            project(p);                                        // :558
             CFDXG_CUDA(cudaMemcpyAsync(E.slot(kCgRsOld), E.slot(kCgRsNew), sizeof(double), cudaMemcpyDeviceToDevice,
                                        ctx->stream));
             rsold = rsnew;
@@ -1514,22 +1785,16 @@ KrylovResult cg_solve(cfdxg_context* ctx, const cfdxg_matrix* A, const double* b
             at_last_replacement = res;
             if (result.first_residual_replacement == 0) result.first_residual_replacement = iter;
             result.last_residual_replacement = iter;
-            E.copy(r, rv);
-            project(r);                                              // :517
-            zero_flags();
-            if (!apply()) return failed(CFDXG_NOT_APPLICABLE, iter, res);
-            dot_check(r, z.get(), kCgRsOld);
-            E.copy(p.get(), z.get());
-            E.fetch(kCgCount);
+            if (!restart_from_residual()) return failed(CFDXG_NOT_APPLICABLE, iter, res);       // :517
             const double replaced = E.host(kCgRsOld);
             if (E.host(kCgZBad) > 0.0 || !std::isfinite(replaced) || !(replaced > 0.0))
                 return failed(CFDXG_NOT_APPLICABLE, iter, res);
             rsold = replaced;
             continue;
         }
-        k_cg_direction<<<gb, kT, 0, ctx->stream>>>(ni, p.get(), z.get(), E.slot(0));
+        k_cg_direction<<<gb, kT, 0, ctx->stream>>>(ni, p, z, E.slot(0));
         check_launch(ctx);
-        project(p.get());                                            // :558
+        project(p);                                            // :558
         CFDXG_CUDA(cudaMemcpyAsync(E.slot(kCgRsOld), E.slot(kCgRsNew), sizeof(double), cudaMemcpyDeviceToDevice,
                                    ctx->stream));
         rsold = rsnew;

@@ -76,8 +76,8 @@ KrylovResult projected_gmres_solve(cfdxg_context* ctx, const cfdxg_matrix* A, co
 // core/linalg/cg_solver.h:45-560 with a preconditioner object (pc, its j
 // argument unused); `setup`, when given, runs after the initial-residual
 // check as the reference's setup_preconditioner and a false return makes the
-// solve NOT_APPLICABLE.  own_diagonal: pc divides by the matrix diagonal and
-// the solve follows the solver's own-diagonal branch (no preconditioner
+// solve NOT_APPLICABLE.  own_diagonal: the matrix diagonal by which pc divides
+// (device, filled by setup); the solve then follows the solver's own-diagonal branch (no preconditioner
 // object, the legacy solve_cg overload, cg_solver.h:591-603) -- its residual
 // replacement rule instead of the adaptive one.
 // null_space: the projected CG of solve_cg(..., NullSpaceProjector) -- a
@@ -87,7 +87,7 @@ KrylovResult projected_gmres_solve(cfdxg_context* ctx, const cfdxg_matrix* A, co
 // 376, 517, 558).
 KrylovResult cg_solve(cfdxg_context* ctx, const cfdxg_matrix* A, const double* b, double* x, int64_t max_iter,
                       double tolerance, const RightPreconditioner& pc, const std::function<bool()>* setup,
-                      bool own_diagonal = false, bool null_space = false);
+                      const double* own_diagonal = nullptr, bool null_space = false);
 
 // Scaled two-pass 2-norm of a device vector (krylov_norm2).
 double device_norm2(cfdxg_context* ctx, const cfdxg_matrix* A, const double* a);

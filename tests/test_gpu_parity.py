@@ -622,3 +622,45 @@ def test_poisson_driver_matches_oracle(ctx, oracle, kind):
         assert out["solution"][cell] == value
         with pytest.raises(ValueError):
             cg.solve_poisson_mixed(mesh, bc, src + 1.0, types)
+
+
+def _chain(n, diag=2.05):
+    """Tridiagonal (-1, diag, -1) of n rows as CSR."""
+    i = np.arange(n)
+    rows = np.concatenate([i, i[1:], i[:-1]])
+    cols = np.concatenate([i, i[:-1], i[1:]])
+    vals = np.concatenate([np.full(n, diag), np.full(2 * (n - 1), -1.0)])
+    order = np.lexsort((cols, rows))
+    ro = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=n))]).astype(np.int64)
+    return ro, cols[order].astype(np.int64), vals[order]
+
+
+@pytest.mark.parametrize("n", [1, 2, 255, 257, 5000, 131073])
+def test_own_diagonal_cg_sizes(ctx, oracle, n):
+    """The own-diagonal CG (one persistent launch) against the oracle's: one
+    row, block remainders, and more rows than the GPU holds threads for; a
+    stop at the iteration limit; a right-hand side outside the range in which
+    the kernel takes the residual's plain squares (the host then decides every
+    iteration; at 1e-145 the products, about 1e-290, are still normal numbers,
+    so the dots of any implementation keep their precision)."""
+    ro, co, va = _chain(n)
+    b = np.random.default_rng(n).standard_normal(n)
+    A = cg.SparseMatrix.from_csr(ctx, ro, co, va)
+    kw = dict(krylov="cg", preconditioner="own_diagonal", tolerance=1e-10)
+    x_ref, rep_ref = oracle.solve_cg(ro, co, va, b, "internal_jacobi", None, tolerance=1e-10)
+    for scale in (1.0, 1e-145):
+        x, rep = cg.solve_linear_system(A, b * scale, **kw)
+        assert rep["status_name"] == "converged" and abs(rep["iterations"] - rep_ref["iterations"]) <= 2
+        assert rel_l2(x / scale, x_ref) <= CG_LONG_TOL
+    if n > 100:
+        x_ref, rep_ref = oracle.solve_cg(ro, co, va, b, "internal_jacobi", None, tolerance=1e-10, max_iterations=5)
+        x, rep = cg.solve_linear_system(A, b, max_iterations=5, **kw)
+        assert rep["iterations"] == 5 and rep["status_name"] == "max_iter_reached" and rep_ref["status"] == 1
+        assert rel_l2(x, x_ref) <= 1e-12     # five updates of FP64 sums in another order
+
+
+def test_own_diagonal_cg_refuses_negative_curvature(ctx):
+    ro, co = np.array([0, 2, 4]), np.array([0, 1, 0, 1])
+    A = cg.SparseMatrix.from_csr(ctx, ro, co, np.array([1.0, 2.0, 2.0, 1.0]))
+    x, rep = cg.solve_linear_system(A, np.array([1.0, -1.0]), krylov="cg", preconditioner="own_diagonal")
+    assert rep["status_name"] == "not_applicable" and np.array_equal(x, np.zeros(2))
