@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "amg_setup.h"
+#include "dense.h"
 #include "device.cuh"
 
 namespace cfdxg {
@@ -62,11 +63,11 @@ struct DevHierarchy {
     DevBuf<float> dense;       // mode 2: the n*n inverse (row-major), formed in FP64, stored FP32
     DevBuf<double> dense64;    // mode 2 with dense_fp64: the same inverse stored FP64
     bool dense_fp64 = false;
-    // the dense inverse's LU solver handle and work arrays, kept for refreshes
+    // the dense inverse's work arrays and LU solver handle, kept for refreshes
+    SpdWorkspace spd;
     std::shared_ptr<void> solver;
     DevBuf<double> lu_a, lu_x, lu_work;
     DevBuf<int> lu_ipiv, lu_info;
-    bool dense_cholesky = false;   // the last inverse came from a Cholesky factor (symmetric level)
     // constant null space: the cycle's mean removals (in index order with
     // reference_order) and the bordered coarsest solve
     bool null_space = false;
