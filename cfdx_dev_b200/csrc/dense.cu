@@ -254,9 +254,9 @@ __global__ void k_symmetry_check(int n, int ld, const double* __restrict__ a, in
     }
 }
 
-// b (n x n, row-major, both triangles) = the negated lower triangle of a
+// b (n x n, row-major with leading dimension ldb, both triangles) = the negated lower triangle of a
 template <class S>
-__global__ void k_negated_symmetric(int n, int ld, const double* __restrict__ a, S* __restrict__ b) {
+__global__ void k_negated_symmetric(int n, int ld, int ldb, const double* __restrict__ a, S* __restrict__ b) {
     __shared__ double tile[32][33];
     const int I = blockIdx.y, J = blockIdx.x;
     if (J > I) return;
@@ -268,9 +268,9 @@ __global__ void k_negated_symmetric(int n, int ld, const double* __restrict__ a,
     __syncthreads();
     for (int r = ty; r < 32; r += 8) {
         const int i = I * 32 + r, j = J * 32 + tx;
-        if (i < n && j <= i) b[static_cast<size_t>(i) * n + j] = static_cast<S>(tile[r][tx]);
+        if (i < n && j <= i) b[static_cast<size_t>(i) * ldb + j] = static_cast<S>(tile[r][tx]);
         const int mi = J * 32 + r, mj = I * 32 + tx;   // the mirrored entry (mi, mj), mj > mi
-        if (mi < n && mj < n && mj > mi) b[static_cast<size_t>(mi) * n + mj] = static_cast<S>(tile[tx][r]);
+        if (mi < n && mj < n && mj > mi) b[static_cast<size_t>(mi) * ldb + mj] = static_cast<S>(tile[tx][r]);
     }
 }
 
@@ -293,7 +293,7 @@ void launch_shared(cfdxg_context* ctx, void (*kern)(double*, int, int, const dou
 }  // namespace
 
 SpdStatus spd_inverse(cfdxg_context* ctx, int n, const int* ro, const int* co, const double* va, SpdWorkspace& w,
-                      float* out32, double* out64) {
+                      int ld_out, float* out32, double* out64) {
     cudaStream_t s = ctx->stream;
     const int tiles = (n + kB - 1) / kB, np = tiles * kB;
     const std::size_t nn = static_cast<std::size_t>(np) * np;
@@ -339,8 +339,8 @@ SpdStatus spd_inverse(cfdxg_context* ctx, int n, const int* ro, const int* co, c
             check_launch(ctx);
         }
     }
-    if (out64) k_negated_symmetric<double><<<dim3(t32, t32), 256, 0, s>>>(n, np, a, out64);
-    else k_negated_symmetric<float><<<dim3(t32, t32), 256, 0, s>>>(n, np, a, out32);
+    if (out64) k_negated_symmetric<double><<<dim3(t32, t32), 256, 0, s>>>(n, np, ld_out, a, out64);
+    else k_negated_symmetric<float><<<dim3(t32, t32), 256, 0, s>>>(n, np, ld_out, a, out32);
     check_launch(ctx);
     int info[2] = {0, 0};
     CFDXG_CUDA(cudaMemcpyAsync(info, w.info.get(), 2 * sizeof(int), cudaMemcpyDeviceToHost, s));

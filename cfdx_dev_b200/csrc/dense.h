@@ -16,10 +16,11 @@ struct SpdWorkspace {
 enum class SpdStatus { kInverted, kNotSymmetric, kNotPositive };
 
 // The inverse of the n x n matrix given by its device CSR (unique columns),
-// row-major into out64, or rounded into out32 when out64 is null.  A matrix
+// row-major (leading dimension ld_out) into out64, or rounded into out32 when
+// out64 is null.  A matrix
 // that is not symmetric to rounding, or not positive definite, is reported
 // and leaves the output undefined.  Synchronises the stream.
 SpdStatus spd_inverse(cfdxg_context* ctx, int n, const int* ro, const int* co, const double* va, SpdWorkspace& w,
-                      float* out32, double* out64);
+                      int ld_out, float* out32, double* out64);
 
 }  // namespace cfdxg

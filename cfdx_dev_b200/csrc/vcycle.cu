@@ -381,26 +381,67 @@ __global__ void k_dense_lu_reference(int n, const int* __restrict__ ro, const in
     for (int i = 0; i < n; ++i) x[i] = static_cast<T>(sol[i]);
 }
 
-// x = Ainv * r, one warp per row: the inverse (formed in FP64) is read as
-// FP32 -- half the bytes of the largest single read of the FP32 cycle -- and
-// the products are summed in FP64.
+// x = Ainv * r: the inverse (formed in FP64) is read as FP32 -- half the bytes
+// of the largest single read of the FP32 cycle -- and the products are summed
+// in FP64.  Bound by reading the inverse (117 MB at 5,401 rows, about 18 us of
+// HBM): a block takes four rows, its threads 16 bytes of each at a time, so
+// that a vector entry is converted once for four rows and enough loads are in
+// flight; the first ones, like every operator, before the wait for r (which
+// carries no __restrict__: an invariant load could be moved above the wait).
+// 21 us at 5,401 rows (5.4 TB/s); a warp per row with 4-byte loads took 33 us
+// (latency).  Rows are padded with zeros to ld entries (16-byte alignment).
+constexpr int kDenseRows = 4;
+
 template <class T, class S>
-__global__ void k_dense_inverse_apply(int n, const S* __restrict__ inv, const T* __restrict__ r,
-                                      T* __restrict__ x, int* status) {
-    pdl_entry();
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (warp >= n) return;
-    double s = 0.0;
-    const S* row = inv + static_cast<size_t>(warp) * n;
-#pragma unroll 4
-    for (int j = lane; j < n; j += 32) s += static_cast<double>(row[j]) * static_cast<double>(r[j]);
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) {
-        x[warp] = static_cast<T>(s);
+__global__ void __launch_bounds__(kT) k_dense_inverse_apply(int n, int ld, const S* __restrict__ inv,
+                                                            const T* r, T* x, int* status) {
+    constexpr int V = 16 / sizeof(S);
+    constexpr int kWarps = kT / 32;
+    __shared__ double part[kWarps][kDenseRows];
+    pdl_trigger();
+    const int row0 = blockIdx.x * kDenseRows;
+    int c = threadIdx.x * V;
+    S m[kDenseRows][V];
+    const auto load = [&](int at) {
+#pragma unroll
+        for (int q = 0; q < kDenseRows; ++q) {
+            const int row = row0 + q < n ? row0 + q : n - 1;
+            *reinterpret_cast<float4*>(m[q]) =
+                __ldg(reinterpret_cast<const float4*>(inv + static_cast<size_t>(row) * ld + at));
+        }
+    };
+    double acc[kDenseRows] = {};
+    if (c < ld) load(c);
+    pdl_wait();
+    while (c < ld) {
+        double rv[V];
+#pragma unroll
+        for (int u = 0; u < V; ++u) rv[u] = c + u < n ? static_cast<double>(r[c + u]) : 0.0;
+#pragma unroll
+        for (int q = 0; q < kDenseRows; ++q)
+#pragma unroll
+            for (int u = 0; u < V; ++u) acc[q] += static_cast<double>(m[q][u]) * rv[u];
+        c += kT * V;
+        if (c < ld) load(c);
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int q = 0; q < kDenseRows; ++q) {
+        for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+        if (lane == 0) part[warp][q] = acc[q];
+    }
+    __syncthreads();
+    if (threadIdx.x < kDenseRows && row0 + static_cast<int>(threadIdx.x) < n) {
+        double s = 0.0;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) s += part[w][threadIdx.x];
+        x[row0 + threadIdx.x] = static_cast<T>(s);
         if (!isfinite(s)) atomicOr(status, kStatusNonFinite);
     }
 }
+
+// entries per stored row of an n x n inverse: a multiple of 16 bytes
+inline int dense_ld(int n) { return (n + 3) & ~3; }
 
 // ---- dense coarse inverse (LU with partial pivoting, cuSOLVER) ----
 // A^T, dense column-major with leading dimension ld (so element (j, i) of the
@@ -423,13 +464,13 @@ __global__ void k_identity(int64_t n, double* x) {
     if (idx < n * n) x[idx] = (idx / n == idx % n) ? 1.0 : 0.0;
 }
 
-// b (n x n) = the leading n x n block of a (row-major, leading dimension ld)
+// b (n x n, leading dimension ldb) = the leading n x n block of a (row-major, leading dimension ld)
 template <class S>
-__global__ void k_dense_block_copy(int n, int ld, const double* __restrict__ a, S* __restrict__ b) {
+__global__ void k_dense_block_copy(int n, int ld, int ldb, const double* __restrict__ a, S* __restrict__ b) {
     const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= static_cast<int64_t>(n) * n) return;
     const int64_t i = idx / n, j = idx % n;
-    b[idx] = static_cast<S>(a[i * ld + j]);
+    b[i * ldb + j] = static_cast<S>(a[i * ld + j]);
 }
 
 #define CFDXG_TPR_SWITCH(tpr, ...)                            \
@@ -702,12 +743,20 @@ void build_dense_inverse_dev(cfdxg_context* ctx, DevHierarchy<T>& d, int n, cons
     const int N = n + (d.null_space ? 1 : 0);
     const std::size_t nn = static_cast<std::size_t>(n) * n;
     const std::size_t NN = static_cast<std::size_t>(N) * N;
-    if (d.dense_fp64) d.dense64.resize(nn);
-    else d.dense.resize(nn);
+    const int ldb = dense_ld(n);
+    const std::size_t stored = static_cast<std::size_t>(n) * ldb;
     cudaStream_t s = ctx->stream;
+    if (d.dense_fp64 && d.dense64.size() != stored) {
+        d.dense64.resize(stored);
+        d.dense64.zero(s);   // the rows' padding stays zero
+    } else if (!d.dense_fp64 && d.dense.size() != stored) {
+        d.dense.resize(stored);
+        d.dense.zero(s);
+    }
     SpdStatus spd = SpdStatus::kNotPositive;
     if (!d.null_space) {
-        spd = spd_inverse(ctx, n, ro, co, va, d.spd, d.dense.get(), d.dense_fp64 ? d.dense64.get() : nullptr);
+        spd = spd_inverse(ctx, n, ro, co, va, d.spd, ldb, d.dense.get(),
+                          d.dense_fp64 ? d.dense64.get() : nullptr);
         if (std::getenv("CFDXG_SETUP_PROFILE") && spd == SpdStatus::kInverted)
             std::fprintf(stderr, "[cfdxg setup] dense coarse inverse of %d rows by symmetric sweeps\n", N);
         if (spd == SpdStatus::kInverted) return;
@@ -750,10 +799,10 @@ void build_dense_inverse_dev(cfdxg_context* ctx, DevHierarchy<T>& d, int n, cons
         throw Error(CFDXG_ERR_CUDA, "dense coarse LU failed");
     CFDXG_CUDA(cudaMemcpyAsync(&host_info, info, sizeof(int), cudaMemcpyDeviceToHost, s));
     if (d.dense_fp64)
-        k_dense_block_copy<double><<<blocks_for(static_cast<int64_t>(nn), kT), kT, 0, s>>>(n, N, x.get(),
+        k_dense_block_copy<double><<<blocks_for(static_cast<int64_t>(nn), kT), kT, 0, s>>>(n, N, ldb, x.get(),
                                                                                          d.dense64.get());
     else
-        k_dense_block_copy<float><<<blocks_for(static_cast<int64_t>(nn), kT), kT, 0, s>>>(n, N, x.get(),
+        k_dense_block_copy<float><<<blocks_for(static_cast<int64_t>(nn), kT), kT, 0, s>>>(n, N, ldb, x.get(),
                                                                                         d.dense.get());
     check_launch(ctx);
     CFDXG_CUDA(cudaStreamSynchronize(s));
@@ -821,11 +870,11 @@ void enqueue_from(cfdxg_context* ctx, DevHierarchy<T>& d, int l) {
         } else if (d.coarse_mode == 2) {
             account((d.dense_fp64 ? 8.0 : 4.0) * L.n * L.n + 2.0 * sizeof(T) * L.n);
             if (d.dense_fp64)
-                launch_pdl(s, k_dense_inverse_apply<T, double>, blocks_for(static_cast<int64_t>(L.n) * 32, kT), kT,
-                           L.n, d.dense64.get(), L.r.get(), L.x.get(), d.status);
+                launch_pdl(s, k_dense_inverse_apply<T, double>, blocks_for(L.n, kDenseRows), kT, L.n, dense_ld(L.n),
+                           d.dense64.get(), L.r.get(), L.x.get(), d.status);
             else
-                launch_pdl(s, k_dense_inverse_apply<T, float>, blocks_for(static_cast<int64_t>(L.n) * 32, kT), kT,
-                           L.n, d.dense.get(), L.r.get(), L.x.get(), d.status);
+                launch_pdl(s, k_dense_inverse_apply<T, float>, blocks_for(L.n, kDenseRows), kT, L.n, dense_ld(L.n),
+                           d.dense.get(), L.r.get(), L.x.get(), d.status);
             check_launch(ctx);
             remove_mean(ctx, d, L.n, L.x.get());
             L.xout = L.x.get();
