@@ -61,9 +61,12 @@ __global__ void k_absmax(int n, const double* __restrict__ a, double* partial, u
     }
 }
 
-// out = scale * sqrt(sum (a_i / scale)^2), NaN on invalid input, 0 when scale == 0.
+// out = scale * sqrt(sum (a_i / scale)^2), NaN on invalid input, 0 when scale == 0;
+// also into *mirror (pinned host memory) when given, which the host reads after
+// a synchronisation instead of copying the slots back.
 __global__ void k_sumsq(int n, const double* __restrict__ a, const double* scale_p,
-                        const double* invalid_p, double* partial, unsigned* ticket, double* out) {
+                        const double* invalid_p, double* partial, unsigned* ticket, double* out,
+                        double* mirror = nullptr) {
     pdl_entry();
     __shared__ double sm[32];
     const double scale = *scale_p;
@@ -86,6 +89,7 @@ __global__ void k_sumsq(int n, const double* __restrict__ a, const double* scale
             else if (!isfinite(t)) r = nan("");
             else r = scale * sqrt(fmax(0.0, t));
             *out = r;
+            if (mirror) *mirror = r;
             *ticket = 0;
         }
     }
@@ -410,6 +414,32 @@ __global__ void k_div(int n, const double* __restrict__ w, const double* d, doub
     if (i < n) v[i] = w[i] / dd;
 }
 
+// The last kernel of an Arnoldi step j: v = w / h_{j+1,j} as k_div, and block 0
+// writes what the host needs of the step -- its scalar slots 0..7, the two
+// Hessenberg columns and the status word -- into the step's pinned mirror
+// (instead of two copies, and of a kernel for the action norm's square root:
+// some 15 us of stream time per step).  action_sq: the slot of the squared
+// action norm, or -1 when slot kAction holds the norm itself.
+__global__ void k_div_publish(int n, const double* __restrict__ w, double* __restrict__ v, const double* slots,
+                              int j, int action_sq, const int* status, double* mirror, int* mirror_status) {
+    pdl_entry();
+    // not __restrict__: an invariant load could be moved above the wait
+    const double dd = slots[kHnext];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (dd > 0.0 && i < n) v[i] = w[i] / dd;
+    if (blockIdx.x != 0) return;
+    for (int q = threadIdx.x; q < 8 + 2 * (j + 1); q += blockDim.x) {
+        const int s = q < 8 ? q : (q < 8 + j + 1 ? kH1 + q - 8 : kH2 + q - 8 - (j + 1));
+        double value = slots[s];
+        if (s == kAction && action_sq >= 0) {
+            const double sq = slots[action_sq];
+            value = isfinite(sq) ? sqrt(sq) : nan("");
+        }
+        mirror[s] = value;
+    }
+    if (threadIdx.x == 0) *mirror_status = *status;
+}
+
 // r = b - A x  (true residual with the FP64 operator)
 __global__ void k_true_residual(int n, const int* __restrict__ ro, const int* __restrict__ co,
                                 const double* __restrict__ va, const double* __restrict__ b,
@@ -434,10 +464,20 @@ __global__ void k_update(int n, const double* __restrict__ x, const double* __re
     out[i] = v;
 }
 
-// *to = sqrt(*from) (NaN when *from is not finite)
-__global__ void k_sqrt_slot(const double* from, double* to) {
-    const double v = *from;
-    *to = isfinite(v) ? sqrt(v) : nan("");
+// The same with the coefficients in the launch's parameters (no copy to the device).
+constexpr int kInlineCoefficients = 64;
+struct Coefficients {
+    double y[kInlineCoefficients];
+};
+__global__ void k_update_inline(int n, const double* x, const double* Z, const __grid_constant__ Coefficients c,
+                                int used, double* out) {
+    pdl_entry();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double v = x[i];
+#pragma unroll 4
+    for (int j = 0; j < used; ++j) v += c.y[j] * Z[static_cast<size_t>(j) * n + i];
+    out[i] = v;
 }
 
 __global__ void k_neg(int n, const double* __restrict__ a, double* __restrict__ b) {
@@ -549,8 +589,13 @@ public:
                                                 slot(kMax), slot(kInvalid));
         check_launch(ctx_);
         launch_pdl(ctx_->stream, k_sumsq, rb(), kT, n_, a, slot(kMax), slot(kInvalid), ctx_->scratch.partial,
-                                               ctx_->scratch.ticket, slot(out));
+                                               ctx_->scratch.ticket, slot(out), ctx_->scratch.host_scalars + out);
         check_launch(ctx_);
+    }
+    // the value of the last norm2 into slot out (synchronises; no copy)
+    double norm_value(int out) {
+        CFDXG_CUDA(cudaStreamSynchronize(ctx_->stream));
+        return host(out);
     }
     void dot(const double* a, const double* b, int out) {
         ProfScope ps(ctx_, "krylov_dot", 2.0 * nb());
@@ -571,7 +616,7 @@ public:
                                                      ctx_->scratch.ticket, slot(kMax), slot(kInvalid));
         check_launch(ctx_);
         launch_pdl(ctx_->stream, k_sumsq, rb(), kT, n_, w, slot(kMax), slot(kInvalid), ctx_->scratch.partial,
-                                               ctx_->scratch.ticket, slot(out));
+                                               ctx_->scratch.ticket, slot(out), static_cast<double*>(nullptr));
         check_launch(ctx_);
     }
     // h[out + i] = v_i . w for i <= j (classical Gram-Schmidt), in chunks
@@ -603,7 +648,7 @@ public:
         if (norm_out >= 0) {
             ProfScope ps(ctx_, "krylov_norm", nb());
             launch_pdl(ctx_->stream, k_sumsq, rb(), kT, n_, w, slot(kMax), slot(kInvalid), ctx_->scratch.partial,
-                                                   ctx_->scratch.ticket, slot(norm_out));
+                                                   ctx_->scratch.ticket, slot(norm_out), static_cast<double*>(nullptr));
             check_launch(ctx_);
         }
     }
@@ -639,10 +684,6 @@ public:
                 check_launch(ctx_);
             }
         });
-    }
-    void sqrt_slot(int from, int to) {
-        k_sqrt_slot<<<1, 1, 0, ctx_->stream>>>(slot(from), slot(to));
-        check_launch(ctx_);
     }
     void axpy_neg(double* w, const double* v, int coef) {
         ProfScope ps(ctx_, "gram_schmidt_axpy", 3.0 * nb());
@@ -723,17 +764,22 @@ public:
                    slot(kMax), slot(kInvalid));
         check_launch(ctx_);
         launch_pdl(ctx_->stream, k_sumsq, b, kT, count, a, slot(kMax), slot(kInvalid), ctx_->scratch.partial,
-                   ctx_->scratch.ticket, slot(out));
+                   ctx_->scratch.ticket, slot(out), ctx_->scratch.host_scalars + out);
         check_launch(ctx_);
     }
     void copy(double* dst, const double* src) {
         CFDXG_CUDA(cudaMemcpyAsync(dst, src, sizeof(double) * n_, cudaMemcpyDeviceToDevice, ctx_->stream));
     }
     void update(const double* x, const double* Z, const std::vector<double>& y, int used, double* out) {
-        if (used > 0)
-            CFDXG_CUDA(cudaMemcpyAsync(slot(kY), y.data(), sizeof(double) * used, cudaMemcpyHostToDevice,
-                                       ctx_->stream));
         ProfScope ps(ctx_, "krylov_update", (used + 2.0) * nb());
+        if (used <= kInlineCoefficients) {
+            Coefficients c{};
+            std::copy_n(y.begin(), used, c.y);
+            launch_pdl(ctx_->stream, k_update_inline, gb(), kT, n_, x, Z, c, used, out);
+            check_launch(ctx_);
+            return;
+        }
+        CFDXG_CUDA(cudaMemcpyAsync(slot(kY), y.data(), sizeof(double) * used, cudaMemcpyHostToDevice, ctx_->stream));
         launch_pdl(ctx_->stream, k_update, gb(), kT, n_, x, Z, slot(kY), used, out);
         check_launch(ctx_);
     }
@@ -752,13 +798,15 @@ public:
         return read_status(ctx_);
     }
     double host(int s) const { return ctx_->scratch.host_scalars[s]; }
-    // Queues the copy of slots [0, count) and of the status word into mirror
-    // buffer k, then marks it with the buffer's event (no synchronisation).
-    void fetch_async(StepMirror& M, int k, int count) {
-        CFDXG_CUDA(cudaMemcpyAsync(M.scalars[k], sc_, sizeof(double) * count, cudaMemcpyDeviceToHost,
-                                   ctx_->stream));
-        CFDXG_CUDA(cudaMemcpyAsync(M.status[k], ctx_->scratch.status, sizeof(int), cudaMemcpyDeviceToHost,
-                                   ctx_->stream));
+    // Ends Arnoldi step j: v = w / h, the step's scalars and the status word
+    // into mirror buffer k, marked by the buffer's event (no synchronisation).
+    void finish_step(StepMirror& M, int k, int j, int action_sq, const double* w, double* v) {
+        {
+            ProfScope ps(ctx_, "krylov_scale", 2.0 * nb());
+            launch_pdl(ctx_->stream, k_div_publish, gb(), kT, n_, w, v, static_cast<const double*>(sc_), j, action_sq,
+                       static_cast<const int*>(ctx_->scratch.status), M.scalars[k], M.status[k]);
+            check_launch(ctx_);
+        }
         CFDXG_CUDA(cudaEventRecord(M.done[k], ctx_->stream));
     }
     double scalar(int s) {   // read one slot
@@ -1067,8 +1115,13 @@ KrylovResult gmres_solve(cfdxg_context* ctx, const cfdxg_matrix* A, const double
     if (n < current_restart) current_restart = static_cast<int>(n);
     if (projection != 0.0) E.set_projection(projection, workspace(ctx, n, current_restart));
 
+    // ||b|| and the initial residual in one wait
+    Workspace* ws = &workspace(ctx, n, current_restart);
     E.norm2(b, kNorm);
-    const double b_norm = E.scalar(kNorm);
+    E.op_residual(b, x, ws->r.get());
+    E.norm2(ws->r.get(), kBeta);
+    double beta = E.norm_value(kBeta);
+    const double b_norm = E.host(kNorm);
     if (!std::isfinite(b_norm)) {
         result.status = CFDXG_DIVERGED;
         return result;
@@ -1109,14 +1162,12 @@ KrylovResult gmres_solve(cfdxg_context* ctx, const cfdxg_matrix* A, const double
     const double rhs_scale = std::max(b_norm, 1e-300);
     const double tol = b_norm == 0.0 ? 0.0 : tolerance * b_norm;
 
-    Workspace* ws = &workspace(ctx, n, current_restart);
     auto true_residual = [&]() {
         E.op_residual(b, x, ws->r.get());
         E.norm2(ws->r.get(), kBeta);
-        return E.scalar(kBeta);
+        return E.norm_value(kBeta);
     };
 
-    double beta = true_residual();
     if (!std::isfinite(beta)) {
         result.status = CFDXG_DIVERGED;
         result.residual = beta;
@@ -1171,7 +1222,8 @@ KrylovResult gmres_solve(cfdxg_context* ctx, const cfdxg_matrix* A, const double
         auto v = [&](int j) { return V + static_cast<size_t>(j) * n; };
         auto z = [&](int j) { return Z + static_cast<size_t>(j) * n; };
 
-        beta = true_residual();
+        // r and beta are those of x: from before the loop, or from the end of
+        // the previous cycle
         if (!std::isfinite(beta)) return fail(CFDXG_DIVERGED);
         if (beta <= tol) break;
         E.div(ws->r.get(), kBeta, v(0));
@@ -1190,11 +1242,12 @@ KrylovResult gmres_solve(cfdxg_context* ctx, const cfdxg_matrix* A, const double
             if (!E.precondition(pc, v(jj), z(jj), jj)) return false;
             E.op(z(jj), ws->w.get());
             double* w = ws->w.get();
+            int action_sq = -1;
             if (controls.classical_gram_schmidt && jj + 1 <= kChunk) {
                 // classical Gram-Schmidt twice in three fused passes; the
-                // action norm comes from the first (slot kH1 + jj + 1)
+                // squared action norm comes from the first (slot kH1 + jj + 1)
                 E.gram_schmidt_cgs2_fused(V, jj + 1, w, ws->mpartial.get());
-                E.sqrt_slot(kH1 + jj + 1, kAction);
+                action_sq = kH1 + jj + 1;
             } else if (controls.classical_gram_schmidt) {
                 // two passes of classical Gram-Schmidt: h = V^T w; w -= V h, twice
                 E.norm2(w, kAction);
@@ -1212,8 +1265,7 @@ KrylovResult gmres_solve(cfdxg_context* ctx, const cfdxg_matrix* A, const double
                 for (int i = 0; i < jj; ++i) E.axpy_dot(w, v(i), kH2 + i, v(i + 1), kH2 + i + 1);
                 E.axpy_norm2(w, v(jj), kH2 + jj, kHnext);
             }
-            E.div(w, kHnext, v(jj + 1));
-            E.fetch_async(mirror, jj & 1, kH2 + jj + 1);
+            E.finish_step(mirror, jj & 1, jj, action_sq, w, v(jj + 1));
             return true;
         };
         // Run-ahead: step j + 1 is queued before step j's results are read
@@ -1363,10 +1415,9 @@ KrylovResult gmres_solve(cfdxg_context* ctx, const cfdxg_matrix* A, const double
             result.max_true_residual = std::max(result.max_true_residual, beta);
         }
         if (!std::isfinite(beta)) return fail(CFDXG_DIVERGED);
-        if (beta < best_residual) {
-            best_residual = beta;
-            E.copy(ws->best.get(), x);
-        }
+        const bool improved = beta < best_residual;
+        if (improved) best_residual = beta;
+        if (improved && !(beta <= tol)) E.copy(ws->best.get(), x);
         if (beta <= tol) {
             result.status = CFDXG_CONVERGED;
             result.iterations = iterations;
