@@ -36,6 +36,14 @@ constexpr int kPatchSymmetry = 3;
 constexpr int kPatchEmpty = 6;
 constexpr int kOtherSide = int(0x80000000u);   // slot record: the cell is the face's neighbour
 
+// The checks of this file's kernels go to two words of pinned host memory
+// (Scratch::face_status): a kernel stores to them only when a check fails, and
+// the host reads them after the call's synchronisation, so a call needs
+// neither a memset before its kernels nor a copy after them.
+__device__ __forceinline__ void raise_status(int* status, int what) {
+    *static_cast<volatile int*>(status + (what == kStatusGeometry ? 1 : 0)) = 1;
+}
+
 struct D3 {
     double x, y, z;
 };
@@ -54,7 +62,7 @@ __global__ void k_face_geometry(int nf, const int* __restrict__ fo, const int* _
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= nf) return;
     const int off = fo[f], nv = fo[f + 1] - off;
-    if (nv < 3) { atomicOr(status, kStatusGeometry); return; }
+    if (nv < 3) { raise_status(status, kStatusGeometry); return; }
     const int v0 = fv[off];
     const D3 p0{px[v0], py[v0], pz[v0]};
     D3 S{0.0, 0.0, 0.0}, awc{0.0, 0.0, 0.0};
@@ -69,7 +77,7 @@ __global__ void k_face_geometry(int nf, const int* __restrict__ fo, const int* _
         tri_area += ta;
     }
     const double area = mag(S);
-    if (!(tri_area > 0.0) || !(area > 0.0) || !isfinite(area)) atomicOr(status, kStatusGeometry);
+    if (!(tri_area > 0.0) || !(area > 0.0) || !isfinite(area)) raise_status(status, kStatusGeometry);
     const D3 c = mul(awc, 1.0 / tri_area);
     fc[f] = c.x; fc[nf + f] = c.y; fc[2 * nf + f] = c.z;
     sf[f] = S.x; sf[nf + f] = S.y; sf[2 * nf + f] = S.z;
@@ -82,7 +90,7 @@ __global__ void k_cell_geometry(int nc, int nf, const int* __restrict__ co, cons
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nc) return;
     const int b = co[c], e = co[c + 1];
-    if (e == b) { atomicOr(status, kStatusGeometry); return; }
+    if (e == b) { raise_status(status, kStatusGeometry); return; }
     bool is_2d = true;
     for (int k = b; k < e; ++k) {
         const int f = cf[k];
@@ -107,13 +115,13 @@ __global__ void k_cell_geometry(int nc, int nf, const int* __restrict__ co, cons
         D3 s = ld3(sf, nf, f);
         if (owner[f] != c) s = mul(s, -1.0);
         const double area = mag(s);
-        if (!(area > 0.0)) atomicOr(status, kStatusGeometry);
+        if (!(area > 0.0)) raise_status(status, kStatusGeometry);
         if (is_2d) sv += area;
         else sv += dot(sub(ld3(fc, nf, f), centre), s);
     }
     if (!is_2d) sv /= 3.0;
     const double v = fabs(sv);
-    if (!(v > 0.0) || !isfinite(v) || !isfinite(sv)) atomicOr(status, kStatusGeometry);
+    if (!(v > 0.0) || !isfinite(v) || !isfinite(sv)) raise_status(status, kStatusGeometry);
     cc[c] = centre.x; cc[nc + c] = centre.y; cc[2 * nc + c] = centre.z;
     if (vol) vol[c] = v;
 }
@@ -140,10 +148,17 @@ struct MeshView {
     const double* geo;   // per-face d, e, Sf . e (face-loop table), null until built
 };
 
+// Per-patch fixed pressure: with up to kInlinePatches patches the table itself
+// travels in the launch's parameters (fixed is null), so a call copies nothing
+// to the device for it (two pageable copies were a third of the 51 us that
+// assembly and product took on a 1,296-cell mesh); else a device table.
+constexpr int kInlinePatches = 32;
 struct BcView {
-    const int* fixed;     // per patch
-    const double* value;  // per patch
-    int n_patches;
+    const int* fixed = nullptr;      // per patch
+    const double* value = nullptr;   // per patch
+    int n_patches = 0;
+    unsigned fixed_mask = 0;
+    double values[kInlinePatches] = {};
 };
 
 // Geometry of one face as the corrector uses it (pressure_face_orthogonal_coefficient,
@@ -168,8 +183,8 @@ __device__ __forceinline__ FaceTerms face_terms(const double* __restrict__ geo, 
     t.d = geo[f];
     t.e = D3{geo[nf + f], geo[2 * nf + f], geo[3 * nf + f]};
     t.oa = geo[4 * nf + f];
-    if (!(t.d > 0.0) || !isfinite(t.d)) atomicOr(status, kStatusGeometry);
-    if (!(t.oa > 0.0) || !isfinite(t.oa)) atomicOr(status, kStatusGeometry);
+    if (!(t.d > 0.0) || !isfinite(t.d)) raise_status(status, kStatusGeometry);
+    if (!(t.oa > 0.0) || !isfinite(t.oa)) raise_status(status, kStatusGeometry);
     t.rfn = dau.x * t.e.x * t.e.x + dau.y * t.e.y * t.e.y + dau.z * t.e.z * t.e.z;
     return t;
 }
@@ -177,7 +192,7 @@ __device__ __forceinline__ FaceTerms face_terms(const double* __restrict__ geo, 
 // :1914-1935 -- rfn (Sf . e) / d
 __device__ __forceinline__ double ortho_coefficient(const FaceTerms& t, int* status) {
     const double coefficient = t.rfn * t.oa / t.d;
-    if (!isfinite(coefficient)) atomicOr(status, kStatusGeometry);
+    if (!isfinite(coefficient)) raise_status(status, kStatusGeometry);
     return coefficient;
 }
 
@@ -186,7 +201,7 @@ __device__ __forceinline__ double nonortho_flux(const FaceTerms& t, D3 S, D3 dau
     const double full = dau.x * gp.x * S.x + dau.y * gp.y * S.y + dau.z * gp.z * S.z;
     const double implicit_flux = t.rfn * dot(gp, t.e) * t.oa;
     const double deferred = full - implicit_flux;
-    if (!isfinite(deferred)) atomicOr(status, kStatusGeometry);
+    if (!isfinite(deferred)) raise_status(status, kStatusGeometry);
     return deferred;
 }
 
@@ -247,6 +262,11 @@ __device__ __forceinline__ void fixed_boundary(const MeshView& m, int f, int o, 
 __device__ __forceinline__ bool boundary_fixed(const MeshView& m, const BcView& bc, int f, double* value) {
     const int p = m.patch[f];
     if (p < 0 || p >= bc.n_patches) return false;
+    if (!bc.fixed) {
+        if (!(bc.fixed_mask >> p & 1u)) return false;
+        *value = bc.values[p];
+        return true;
+    }
     if (!bc.fixed[p]) return false;
     *value = bc.value[p];
     return true;
@@ -257,7 +277,7 @@ __device__ __forceinline__ bool boundary_fixed(const MeshView& m, const BcView& 
 // the face, the side and the other cell in one load, and the interpolation
 // weight of the cell's side comes from the table (no face-centre or
 // cell-centre reads, no square roots or divisions per call).
-__global__ void k_gauss_gradient(MeshView m, BcView bc, const int2* __restrict__ rec,
+__global__ void k_gauss_gradient(MeshView m, const __grid_constant__ BcView bc, const int2* __restrict__ rec,
                                  const double* __restrict__ wslot, const double* __restrict__ p, double* grad,
                                  int* status) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -285,7 +305,7 @@ __global__ void k_gauss_gradient(MeshView m, BcView bc, const int2* __restrict__
     }
     const double invV = 1.0 / m.vol[c];
     const double gx = sum.x * invV, gy = sum.y * invV, gz = sum.z * invV;
-    if (!isfinite(gx) || !isfinite(gy) || !isfinite(gz)) atomicOr(status, kStatusNonFinite);
+    if (!isfinite(gx) || !isfinite(gy) || !isfinite(gz)) raise_status(status, kStatusNonFinite);
     grad[c] = gx; grad[m.nc + c] = gy; grad[2 * m.nc + c] = gz;
 }
 
@@ -369,7 +389,7 @@ __device__ __forceinline__ void assemble_cell(const MeshView& m, const BcView& b
 // One thread per cell; tetrahedra and hexahedra take the unrolled forms.
 // Capped at 64 registers (eight 128-thread blocks per SM instead of six at
 // 80): 180 instead of 192 us at 64^3, despite a few spilled registers.
-__global__ void __launch_bounds__(kT, 8) k_pressure_assembly(MeshView m, BcView bc, const int2* __restrict__ rec,
+__global__ void __launch_bounds__(kT, 8) k_pressure_assembly(MeshView m, const __grid_constant__ BcView bc, const int2* __restrict__ rec,
                                     const double* __restrict__ U, const double* __restrict__ rau,
                                     const double* __restrict__ p, const double* __restrict__ grad, double rho,
                                     const int* __restrict__ slot, const int* __restrict__ diag_pos,
@@ -378,7 +398,7 @@ __global__ void __launch_bounds__(kT, 8) k_pressure_assembly(MeshView m, BcView 
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.nc) return;
     const int beg = m.co[c], nfc = m.co[c + 1] - beg;
-    if (nfc > kMaxCellFaces) { atomicOr(status, kStatusGeometry); return; }
+    if (nfc > kMaxCellFaces) { raise_status(status, kStatusGeometry); return; }
     if (nfc == 4)
         assemble_cell<4>(m, bc, rec, U, rau, p, grad, rho, slot, diag_pos, values, b, phi_out, status, c, beg, nfc);
     else if (nfc == 6)
@@ -388,7 +408,7 @@ __global__ void __launch_bounds__(kT, 8) k_pressure_assembly(MeshView m, BcView 
 }
 
 // make_rhie_chow_mass_flux (:2064-2217), HBYA_PREDICTOR, zero-gradient velocity boundaries
-__global__ void k_rhie_chow_flux(MeshView m, BcView bc, const double* __restrict__ U,
+__global__ void k_rhie_chow_flux(MeshView m, const __grid_constant__ BcView bc, const double* __restrict__ U,
                                  const double* __restrict__ rau, const double* __restrict__ p,
                                  const double* __restrict__ grad, double rho, double* __restrict__ flux,
                                  int* status) {
@@ -454,7 +474,7 @@ __global__ void k_slot_weights(int nc, int nf, const int* __restrict__ co, const
         const D3 fcv = ld3(fc, nf, r.x & 0x7fffffff);
         const double dc = mag(sub(fcv, ccv));
         const double dn = mag(sub(ld3(cc, nc, r.y), fcv));
-        if (!(dc + dn > 0.0)) atomicOr(status, kStatusGeometry);
+        if (!(dc + dn > 0.0)) raise_status(status, kStatusGeometry);
         w[k] = dn / (dc + dn);
     }
 }
@@ -474,16 +494,16 @@ __global__ void k_diffusion_assembly(MeshView m, const double* __restrict__ bcv,
         const int f = m.cf[beg + k];
         const int o = m.owner[f], n = m.neigh[f];
         const double area = mag(ld3(m.sf, m.nf, f));
-        if (!(area > 0.0) || !isfinite(area)) atomicOr(status, kStatusGeometry);
+        if (!(area > 0.0) || !isfinite(area)) raise_status(status, kStatusGeometry);
         if (n >= 0) {
             const double d = mag(sub(ld3(m.cc, m.nc, n), ld3(m.cc, m.nc, o)));
-            if (!(d > 2.220446049250313080847e-16) || !isfinite(d)) atomicOr(status, kStatusGeometry);
+            if (!(d > 2.220446049250313080847e-16) || !isfinite(d)) raise_status(status, kStatusGeometry);
             const double g = gamma * area / d;
             diag += g;
             values[slot[beg + k]] = 0.0 + (-g);
         } else if (isfinite(bcv[f])) {
             const double d = mag(sub(ld3(m.fc, m.nf, f), ld3(m.cc, m.nc, o)));
-            if (!(d > 2.220446049250313080847e-16) || !isfinite(d)) atomicOr(status, kStatusGeometry);
+            if (!(d > 2.220446049250313080847e-16) || !isfinite(d)) raise_status(status, kStatusGeometry);
             const double g = gamma * area / d;
             if (!bct || bct[f] == 0) {
                 diag += g;
@@ -519,7 +539,7 @@ __global__ void k_build_hbya(int n, const int* __restrict__ ro, const int* __res
     }
     const double v = rau[t] * h;
     hbya[t] = v;
-    if (!isfinite(v)) atomicOr(status, kStatusNonFinite);
+    if (!isfinite(v)) raise_status(status, kStatusNonFinite);
 }
 
 MeshView view(const cfdxg_mesh* m) {
@@ -532,7 +552,7 @@ MeshView view(const cfdxg_mesh* m) {
 void launch_gradient(cfdxg_context* ctx, const cfdxg_mesh* m, const MeshView& mv, const BcView& bc,
                      const double* p, double* grad) {
     k_gauss_gradient<<<blocks_for(m->n_cells, kT), kT, 0, ctx->stream>>>(mv, bc, m->slot_rec.get(), m->slot_w.get(),
-                                                                        p, grad, ctx->scratch.status);
+                                                                        p, grad, ctx->scratch.face_status);
     check_launch(ctx);
 }
 
@@ -553,7 +573,7 @@ void build_face_tables(cfdxg_context* ctx, cfdxg_mesh* m) {
     m->slot_w.resize(static_cast<std::size_t>(nslot));
     k_slot_weights<<<blocks_for(nc, kT), kT, 0, ctx->stream>>>(
         static_cast<int>(nc), static_cast<int>(nf), m->cell_off.get(), m->slot_rec.get(), m->face_centre.get(),
-        m->cell_centre.get(), m->slot_w.get(), ctx->scratch.status);
+        m->cell_centre.get(), m->slot_w.get(), ctx->scratch.face_status);
     check_launch(ctx);
     m->face_geo.resize(static_cast<std::size_t>(kFaceTermArrays) * nf);
     k_face_terms<<<blocks_for(nf, kT), kT, 0, ctx->stream>>>(static_cast<int>(nf), static_cast<int>(nc),
@@ -582,8 +602,23 @@ void require_geometry(const cfdxg_mesh* m) {
     if (!m->geometry_ready) throw Error(CFDXG_ERR_NOT_READY, "geometry not built: call cfdxg_geometry_build");
 }
 
+// The status words before a call's kernels (none of the context is in flight:
+// every call that writes them ends with check_device_status) ...
+void clear_face_status(cfdxg_context* ctx) {
+    volatile int* w = ctx->scratch.face_status;
+    w[0] = 0;
+    w[1] = 0;
+}
+
+// ... and after them: waits for the stream, then reads.
+int read_face_status(cfdxg_context* ctx) {
+    CFDXG_CUDA(cudaStreamSynchronize(ctx->stream));
+    const volatile int* w = ctx->scratch.face_status;
+    return (w[0] ? kStatusNonFinite : 0) | (w[1] ? kStatusGeometry : 0);
+}
+
 void check_device_status(cfdxg_context* ctx, const char* what) {
-    const int st = read_status(ctx);
+    const int st = read_face_status(ctx);
     if (st & kStatusGeometry) throw Error(CFDXG_ERR_GEOMETRY, std::string(what) + ": invalid or inconsistent face geometry");
     if (st & kStatusNonFinite) throw Error(CFDXG_ERR_NONFINITE, std::string(what) + ": non-finite result");
 }
@@ -745,8 +780,8 @@ extern "C" int cfdxg_geometry_build(cfdxg_context* ctx, cfdxg_mesh* m) {
     m->face_sf.resize(3 * static_cast<size_t>(nf));
     m->cell_centre.resize(3 * static_cast<size_t>(nc));
     m->cell_volume.resize(nc);
-    clear_status(ctx);
-    int* st = ctx->scratch.status;
+    clear_face_status(ctx);
+    int* st = ctx->scratch.face_status;
     k_face_geometry<<<blocks_for(nf, kT), kT, 0, s>>>(nf, m->face_off.get(), m->face_vert.get(), m->px.get(),
                                                       m->py.get(), m->pz.get(), m->face_centre.get(),
                                                       m->face_sf.get(), st);
@@ -800,10 +835,10 @@ extern "C" int cfdxg_assemble_cell_diffusion(cfdxg_context* ctx, cfdxg_mesh* m, 
     In<int32_t> bt(ctx, bc_types, bc_types ? nf : 0, mem);
     Out<double> r(ctx, rhs, nc, mem);
     std::unique_ptr<cfdxg_matrix> A(new_pattern_matrix(ctx, m));
-    clear_status(ctx);
+    clear_face_status(ctx);
     k_diffusion_assembly<<<blocks_for(nc, kT), kT, 0, ctx->stream>>>(view(m), bv.get(), bt.get(), gamma, src.get(),
                                                                      m->pattern.d_slot.get(), m->pattern.d_diag.get(),
-                                                                     A->va.get(), r.get(), ctx->scratch.status);
+                                                                     A->va.get(), r.get(), ctx->scratch.face_status);
     check_launch(ctx);
     r.finish();
     check_device_status(ctx, "assemble_cell_diffusion_matrix");
@@ -814,9 +849,19 @@ extern "C" int cfdxg_assemble_cell_diffusion(cfdxg_context* ctx, cfdxg_mesh* m, 
 }
 
 namespace {
-// Per-patch fixed-pressure table in the mesh's own device buffers.
+// Per-patch fixed-pressure table: in the view itself, or, of more than
+// kInlinePatches patches, in the mesh's own device buffers.
 BcView make_bc(cfdxg_context* ctx, cfdxg_mesh* m, const int32_t* fixed, const double* value) {
-    const int np = std::max<int>(1, m->n_patches);
+    BcView view;
+    view.n_patches = static_cast<int>(m->n_patches);
+    if (m->n_patches <= kInlinePatches) {
+        for (int p = 0; p < m->n_patches; ++p) {
+            if (fixed && fixed[p]) view.fixed_mask |= 1u << p;
+            view.values[p] = value ? value[p] : 0.0;
+        }
+        return view;
+    }
+    const int np = static_cast<int>(m->n_patches);
     std::vector<int> f(np, 0);
     std::vector<double> v(np, 0.0);
     for (int p = 0; p < m->n_patches; ++p) {
@@ -825,7 +870,9 @@ BcView make_bc(cfdxg_context* ctx, cfdxg_mesh* m, const int32_t* fixed, const do
     }
     m->bc_fixed.upload(f, ctx->stream);
     m->bc_value.upload(v, ctx->stream);
-    return {m->bc_fixed.get(), m->bc_value.get(), static_cast<int>(m->n_patches)};
+    view.fixed = m->bc_fixed.get();
+    view.value = m->bc_value.get();
+    return view;
 }
 
 double* gradient_scratch(cfdxg_mesh* m) {
@@ -845,7 +892,7 @@ extern "C" int cfdxg_gauss_gradient(cfdxg_context* ctx, cfdxg_mesh* m, const dou
     const BcView bc = make_bc(ctx, m, fixed, value);
     In<double> pin(ctx, p, nc, mem);
     Out<double> g(ctx, grad, 3 * nc, mem);
-    clear_status(ctx);
+    clear_face_status(ctx);
     {
         ProfScope ps(ctx, "gauss_gradient", gradient_bytes(m));
         launch_gradient(ctx, m, view(m), bc, pin.get(), g.get());
@@ -884,7 +931,7 @@ extern "C" int cfdxg_assemble_pressure_correction(cfdxg_context* ctx, cfdxg_mesh
     } else if (A->mesh != m) {
         throw Error(CFDXG_ERR_INVALID_ARGUMENT, "matrix was not assembled on this mesh");
     }
-    clear_status(ctx);
+    clear_face_status(ctx);
     const MeshView mv = view(m);
     {
         ProfScope ps(ctx, "gauss_gradient", gradient_bytes(m));
@@ -895,7 +942,7 @@ extern "C" int cfdxg_assemble_pressure_correction(cfdxg_context* ctx, cfdxg_mesh
         k_pressure_assembly<<<blocks_for(nc, kT), kT, 0, ctx->stream>>>(mv, bc, m->slot_rec.get(), U.get(), rau.get(),
                                                                         pin.get(), g, rho, m->pattern.d_slot.get(),
                                                                         m->pattern.d_diag.get(), A->va.get(),
-                                                                        bout.get(), phi.get(), ctx->scratch.status);
+                                                                        bout.get(), phi.get(), ctx->scratch.face_status);
         check_launch(ctx);
     }
     bout.finish();
@@ -923,7 +970,7 @@ extern "C" int cfdxg_rhie_chow_flux(cfdxg_context* ctx, cfdxg_mesh* m, const dou
     In<double> U(ctx, HbyA, 3 * nc, mem), rau(ctx, rAU, 3 * nc, mem), pin(ctx, p, nc, mem);
     Out<double> fl(ctx, flux, nf, mem);
     double* g = gradient_scratch(m);
-    clear_status(ctx);
+    clear_face_status(ctx);
     const MeshView mv = view(m);
     {
         ProfScope ps(ctx, "gauss_gradient", gradient_bytes(m));
@@ -932,7 +979,7 @@ extern "C" int cfdxg_rhie_chow_flux(cfdxg_context* ctx, cfdxg_mesh* m, const dou
     {
         ProfScope ps(ctx, "rhie_chow_flux", flux_bytes(m));
         k_rhie_chow_flux<<<blocks_for(nf, kT), kT, 0, ctx->stream>>>(mv, bc, U.get(), rau.get(), pin.get(),
-                                                                     g, rho, fl.get(), ctx->scratch.status);
+                                                                     g, rho, fl.get(), ctx->scratch.face_status);
         check_launch(ctx);
     }
     fl.finish();
@@ -1033,14 +1080,17 @@ extern "C" int cfdxg_rhie_chow_flux_noalloc(cfdxg_context* ctx, cfdxg_mesh* m, c
         t.value[k] = value ? value[k] : 0.0;
     }
     const int64_t nc = m->n_cells, nf = m->n_faces;
-    clear_status(ctx);
+    clear_face_status(ctx);
     k_fill_patch_table<<<1, kNoAllocMaxPatches, 0, ctx->stream>>>(t, tfixed, tvalue);
     check_launch(ctx);
-    const BcView bc{tfixed, tvalue, static_cast<int>(m->n_patches)};
+    BcView bc;
+    bc.fixed = tfixed;
+    bc.value = tvalue;
+    bc.n_patches = static_cast<int>(m->n_patches);
     const MeshView mv = view(m);
     launch_gradient(ctx, m, mv, bc, p, grad);
     k_rhie_chow_flux<<<blocks_for(nf, kT), kT, 0, ctx->stream>>>(mv, bc, HbyA, rAU, p, grad, rho, flux,
-                                                                 ctx->scratch.status);
+                                                                 ctx->scratch.face_status);
     check_launch(ctx);
     check_device_status(ctx, "make_rhie_chow_mass_flux (no-alloc)");
     ctx->error.clear();
@@ -1069,7 +1119,7 @@ extern "C" int cfdxg_build_hbya(cfdxg_context* ctx, cfdxg_mesh* m, const cfdxg_m
     In<double> b(ctx, rhs, 3 * nc, mem), u(ctx, U, 3 * nc, mem), gp(ctx, gradp, 3 * nc, mem),
         rau(ctx, rAU, 3 * nc, mem);
     Out<double> out(ctx, HbyA, 3 * nc, mem);
-    clear_status(ctx);
+    clear_face_status(ctx);
     {
         // momentum values of three components + pattern, rhs/U/gradp/rAU reads, V, HbyA write
         ProfScope ps(ctx, "build_hbya", 3.0 * 8.0 * momentum[0]->nnz + 4.0 * (nc + 1) + 4.0 * momentum[0]->nnz +
@@ -1077,11 +1127,11 @@ extern "C" int cfdxg_build_hbya(cfdxg_context* ctx, cfdxg_mesh* m, const cfdxg_m
         k_build_hbya<<<blocks_for(3 * nc, kT), kT, 0, ctx->stream>>>(
             static_cast<int>(nc), momentum[0]->ro.get(), momentum[0]->co.get(), momentum[0]->va.get(),
             momentum[1]->va.get(), momentum[2]->va.get(), b.get(), u.get(), gp.get(), m->cell_volume.get(),
-            rau.get(), out.get(), ctx->scratch.status);
+            rau.get(), out.get(), ctx->scratch.face_status);
         check_launch(ctx);
     }
     out.finish();
-    const int st = read_status(ctx);
+    const int st = read_face_status(ctx);
     if (st & kStatusNonFinite) throw Error(CFDXG_ERR_NONFINITE, "solve_steady_incompressible: non-finite HbyA");
     ctx->error.clear();
     return CFDXG_OK;

@@ -228,6 +228,7 @@ extern "C" int cfdxg_context_create(int32_t device, cfdxg_context** out) {
         CFDXG_CUDA(cudaMemset(ctx->scratch.status, 0, sizeof(int)));
         CFDXG_CUDA(cudaMallocHost(&ctx->scratch.host_scalars, sizeof(double) * 4096));
         CFDXG_CUDA(cudaMallocHost(&ctx->scratch.host_status, sizeof(int)));
+        CFDXG_CUDA(cudaMallocHost(&ctx->scratch.face_status, 2 * sizeof(int)));
     } catch (const Error& e) {
         const int code = e.code;
         cfdxg_context_destroy(ctx);
@@ -250,6 +251,7 @@ extern "C" int cfdxg_context_destroy(cfdxg_context* ctx) {
     if (ctx->scratch.status) cudaFree(ctx->scratch.status);
     if (ctx->scratch.host_scalars) cudaFreeHost(ctx->scratch.host_scalars);
     if (ctx->scratch.host_status) cudaFreeHost(ctx->scratch.host_status);
+    if (ctx->scratch.face_status) cudaFreeHost(ctx->scratch.face_status);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return CFDXG_OK;

@@ -70,6 +70,7 @@ struct Scratch {
     int* status = nullptr;          // device error word
     double* host_scalars = nullptr; // pinned mirror of `scalars`
     int* host_status = nullptr;     // pinned
+    int* face_status = nullptr;     // pinned, written by the face-loop kernels: non-finite, geometry
 };
 
 // Reusable device staging buffers for host-memory arguments (avoids a
