@@ -320,20 +320,60 @@ __device__ __forceinline__ double pick_slot(const double (&a)[NF], int k) {
     return v;
 }
 
-// Pressure-corrector block (:8048-8181) of cell c: its CSR row and b.
-// Continuity is summed in cell-face order, the diagonal and the fixed-pressure
-// boundary terms in global face order (the per-cell sorted permutation cs), as
-// the reference sums them.  NF > 0: a cell of exactly NF faces, every loop
-// unrolled and the face coefficients in registers; NF = 0: up to
-// kMaxCellFaces faces, the coefficients in local memory.
+// The corrector block (:8048-8181) in two kernels.  Every face is formed once,
+// by the face's thread, whose face arrays are read coalesced and whose owner
+// reads nearly so, and leaves a 32-byte record (one sector) for its two cells:
+//   phi        the mass flux of HbyA;
+//   rc         interior: the Rhie-Chow pressure flux; fixed-pressure
+//              boundary: the source of the owner's right-hand side;
+//   coefficient  rho times the face coefficient;
+//   fixed      1 on a fixed-pressure boundary face, else 0.
+// The cell-centric form, which formed each face from both of its cells, was
+// bound by the latency of some 64 sector look-ups per cell: 179 us at 1,572,864
+// tetrahedra, against 153 us for the two kernels (one launch, half a
+// microsecond, more on a mesh of a thousand cells).
+struct __align__(16) FaceRecord {
+    double phi, rc, coefficient, fixed;
+};
+
+__global__ void __launch_bounds__(kT) k_corrector_faces(MeshView m, const __grid_constant__ BcView bc,
+                                                        const double* __restrict__ U, const double* __restrict__ rau,
+                                                        const double* __restrict__ p, const double* __restrict__ grad,
+                                                        double rho, FaceRecord* __restrict__ faces,
+                                                        double* __restrict__ phi_out, int* status) {
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= m.nf) return;
+    const int o = m.owner[f], n = m.neigh[f];
+    FaceRecord r{mass_flux(m, f, o, n, U, rho), 0.0, 0.0, 0.0};
+    if (n >= 0) {
+        double ic;
+        r.rc = rc_internal(m, f, o, n, p, grad, rau, rho, &ic, status);
+        r.coefficient = rho * ic;
+    } else {
+        double value;
+        if (boundary_fixed(m, bc, f, &value)) {
+            double bcoef;
+            fixed_boundary(m, f, o, p, grad, rau, rho, value, &bcoef, &r.rc, status);
+            r.coefficient = rho * bcoef;
+            r.fixed = 1.0;
+        }
+    }
+    double2* out = reinterpret_cast<double2*>(faces + f);
+    out[0] = make_double2(r.phi, r.rc);
+    out[1] = make_double2(r.coefficient, r.fixed);
+    if (phi_out) phi_out[f] = r.phi;
+}
+
+// Cell c: its CSR row and b from its faces' records.  Continuity is summed in
+// cell-face order, the diagonal and the fixed-pressure boundary terms in
+// global face order (the per-cell sorted permutation cs), as the reference
+// sums them.  NF > 0: a cell of exactly NF faces, every loop unrolled and the
+// records in registers; NF = 0: up to kMaxCellFaces faces, in local memory.
 template <int NF>
-__device__ __forceinline__ void assemble_cell(const MeshView& m, const BcView& bc, const int2* __restrict__ rec,
-                                              const double* __restrict__ U, const double* __restrict__ rau,
-                                              const double* __restrict__ p, const double* __restrict__ grad,
-                                              double rho, const int* __restrict__ slot,
-                                              const int* __restrict__ diag_pos, double* __restrict__ values,
-                                              double* __restrict__ b, double* __restrict__ phi_out, int* status,
-                                              int c, int beg, int nfc) {
+__device__ __forceinline__ void corrector_cell(const MeshView& m, const int2* __restrict__ rec,
+                                               const FaceRecord* __restrict__ faces, const int* __restrict__ slot,
+                                               const int* __restrict__ diag_pos, double* __restrict__ values,
+                                               double* __restrict__ b, int c, int beg, int nfc) {
     constexpr int kCap = NF > 0 ? NF : kMaxCellFaces;
     const int n_slots = NF > 0 ? NF : nfc;
     double coeff[kCap];
@@ -342,19 +382,16 @@ __device__ __forceinline__ void assemble_cell(const MeshView& m, const BcView& b
 #pragma unroll
     for (int k = 0; k < n_slots; ++k) {
         const int2 r = rec[beg + k];
-        const int f = r.x & 0x7fffffff;
+        const double2* face = reinterpret_cast<const double2*>(faces + (r.x & 0x7fffffff));
+        const double2 flux = __ldg(face);
+        const double coefficient = __ldg(&face[1].x);
         const bool own = r.x >= 0;
-        const int o = own ? c : r.y, n = own ? r.y : c;
-        const double phi = mass_flux(m, f, o, n, U, rho);
-        if (phi_out && own) phi_out[f] = phi;
-        cont += own ? phi : -phi;
+        cont += own ? flux.x : -flux.x;
         coeff[k] = 0.0;
         if (r.y >= 0) {
             interior |= 1u << k;
-            double ic;
-            const double rc = rc_internal(m, f, o, n, p, grad, rau, rho, &ic, status);
-            cont += own ? -rc : rc;
-            coeff[k] = rho * ic;
+            cont += own ? -flux.y : flux.y;
+            coeff[k] = coefficient;
         }
     }
     double diag = 0.0;
@@ -370,13 +407,10 @@ __device__ __forceinline__ void assemble_cell(const MeshView& m, const BcView& b
         for (int q = 0; q < n_slots; ++q) {
             const int k = m.cs[beg + q];
             if (interior >> k & 1u) continue;
-            const int f = rec[beg + k].x & 0x7fffffff;
-            double value;
-            if (!boundary_fixed(m, bc, f, &value)) continue;
-            double bcoef, source;
-            fixed_boundary(m, f, c, p, grad, rau, rho, value, &bcoef, &source, status);
-            acc += rho * bcoef;
-            bb += source;
+            const FaceRecord face = faces[rec[beg + k].x & 0x7fffffff];
+            if (face.fixed == 0.0) continue;
+            acc += face.coefficient;
+            bb += face.rc;
         }
     }
     values[diag_pos[c]] = acc;
@@ -387,24 +421,19 @@ __device__ __forceinline__ void assemble_cell(const MeshView& m, const BcView& b
 }
 
 // One thread per cell; tetrahedra and hexahedra take the unrolled forms.
-// Capped at 64 registers (eight 128-thread blocks per SM instead of six at
-// 80): 180 instead of 192 us at 64^3, despite a few spilled registers.
-__global__ void __launch_bounds__(kT, 8) k_pressure_assembly(MeshView m, const __grid_constant__ BcView bc, const int2* __restrict__ rec,
-                                    const double* __restrict__ U, const double* __restrict__ rau,
-                                    const double* __restrict__ p, const double* __restrict__ grad, double rho,
-                                    const int* __restrict__ slot, const int* __restrict__ diag_pos,
-                                    double* __restrict__ values, double* __restrict__ b,
-                                    double* __restrict__ phi_out, int* status) {
+__global__ void __launch_bounds__(kT) k_pressure_assembly(MeshView m, const int2* __restrict__ rec,
+                                                          const FaceRecord* __restrict__ faces,
+                                                          const int* __restrict__ slot,
+                                                          const int* __restrict__ diag_pos,
+                                                          double* __restrict__ values, double* __restrict__ b,
+                                                          int* status) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.nc) return;
     const int beg = m.co[c], nfc = m.co[c + 1] - beg;
     if (nfc > kMaxCellFaces) { raise_status(status, kStatusGeometry); return; }
-    if (nfc == 4)
-        assemble_cell<4>(m, bc, rec, U, rau, p, grad, rho, slot, diag_pos, values, b, phi_out, status, c, beg, nfc);
-    else if (nfc == 6)
-        assemble_cell<6>(m, bc, rec, U, rau, p, grad, rho, slot, diag_pos, values, b, phi_out, status, c, beg, nfc);
-    else
-        assemble_cell<0>(m, bc, rec, U, rau, p, grad, rho, slot, diag_pos, values, b, phi_out, status, c, beg, nfc);
+    if (nfc == 4) corrector_cell<4>(m, rec, faces, slot, diag_pos, values, b, c, beg, nfc);
+    else if (nfc == 6) corrector_cell<6>(m, rec, faces, slot, diag_pos, values, b, c, beg, nfc);
+    else corrector_cell<0>(m, rec, faces, slot, diag_pos, values, b, c, beg, nfc);
 }
 
 // make_rhie_chow_mass_flux (:2064-2217), HBYA_PREDICTOR, zero-gradient velocity boundaries
@@ -879,6 +908,12 @@ double* gradient_scratch(cfdxg_mesh* m) {
     m->grad_scratch.resize(3 * static_cast<std::size_t>(m->n_cells));
     return m->grad_scratch.get();
 }
+
+// The corrector's face records (kept with the mesh after the first assembly).
+double* face_scratch(cfdxg_mesh* m) {
+    m->face_scratch.resize(4 * static_cast<std::size_t>(m->n_faces));
+    return m->face_scratch.get();
+}
 }  // namespace
 
 extern "C" int cfdxg_gauss_gradient(cfdxg_context* ctx, cfdxg_mesh* m, const double* p, const int32_t* fixed,
@@ -939,10 +974,14 @@ extern "C" int cfdxg_assemble_pressure_correction(cfdxg_context* ctx, cfdxg_mesh
     }
     {
         ProfScope ps(ctx, "pressure_assembly", assembly_bytes(m, A->nnz));
-        k_pressure_assembly<<<blocks_for(nc, kT), kT, 0, ctx->stream>>>(mv, bc, m->slot_rec.get(), U.get(), rau.get(),
-                                                                        pin.get(), g, rho, m->pattern.d_slot.get(),
+        FaceRecord* faces = reinterpret_cast<FaceRecord*>(face_scratch(m));
+        k_corrector_faces<<<blocks_for(nf, kT), kT, 0, ctx->stream>>>(mv, bc, U.get(), rau.get(), pin.get(), g, rho,
+                                                                      faces, phi.get(), ctx->scratch.face_status);
+        check_launch(ctx);
+        k_pressure_assembly<<<blocks_for(nc, kT), kT, 0, ctx->stream>>>(mv, m->slot_rec.get(), faces,
+                                                                        m->pattern.d_slot.get(),
                                                                         m->pattern.d_diag.get(), A->va.get(),
-                                                                        bout.get(), phi.get(), ctx->scratch.face_status);
+                                                                        bout.get(), ctx->scratch.face_status);
         check_launch(ctx);
     }
     bout.finish();

@@ -108,7 +108,7 @@ struct cfdxg_mesh {
     // per-call boundary table and gradient scratch, kept so the face-loop entry
     // points neither allocate nor free device memory after their first call
     cfdxg::DevBuf<int> bc_fixed;
-    cfdxg::DevBuf<double> bc_value, grad_scratch;
+    cfdxg::DevBuf<double> bc_value, grad_scratch, face_scratch;
     // host copies needed by the pattern build
     std::vector<int64_t> h_owner, h_neigh, h_cell_off, h_cell_face;
     std::vector<int32_t> h_patch_types;
