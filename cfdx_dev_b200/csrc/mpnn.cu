@@ -314,20 +314,21 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 
 __device__ __forceinline__ uint32_t ld32(const __nv_bfloat16* p) { return *reinterpret_cast<const uint32_t*>(p); }
 
-constexpr int kUPad = 2 * F + 8;   // 72 bf16 per row: 144 B, keeps 4-byte loads conflict-light
-constexpr int kW2Pad = F + 8;
-
-// Inference round, gather-optimised.  A warp owns 16 consecutive cells.  Their
-// off-diagonal couplings are one contiguous CSR segment, staged in shared
-// memory with coalesced loads; the gather then runs 8 lanes per cell (each
-// lane a 16-byte quarter-row of 4 features) over 4 cells at a time, with four
-// neighbour rows in flight per lane.  [h, a] goes to shared memory as BF16 for
-// the two tensor-core layers; the FP32 h stays in shared memory for the
-// residual update.
+// Inference rounds.  A warp owns 16 consecutive cells, rows g and g + 8 (g =
+// lane / 4) of the MMA tile, and the four lanes of a row (t = lane % 4) gather
+// its neighbours' states 16 bytes each: features 8 t .. 8 t + 7.  Contractions
+// do not depend on the order of their terms, so the features are numbered
+// within the MMA's k slots as the gather delivers them -- slot pairs (2 t, 2 t
+// + 1) and (2 t + 8, 2 t + 9) of k block q hold features 8 t + 4 q .. + 3 --
+// and the output columns so that a lane ends with features 8 t .. 8 t + 7 of
+// its two rows: [h, a] is the A operand straight from registers, the new state
+// leaves in 16-byte stores, and nothing passes through shared memory.  The
+// weights stay in registers (48) over the warp's tiles, and a tile's couplings
+// are loaded one tile ahead.  Bound by the latency of the L2 gathers (some 400
+// bytes a cell and round): four rounds at 663,552 cells take 250 us; with 8
+// lanes of 8 bytes per row and the operands staged in shared memory 330.
 constexpr int kTileCells = 16;
-constexpr int kSegCap = 128;           // staged couplings per 16-cell tile
-constexpr int kRoundWarps = 6;
-constexpr int kRoundThreads = 32 * kRoundWarps;
+constexpr int kRoundThreads = 128;
 
 // x_i = [r_i / s, f_V, f_P, f_D] packed as one float4 per cell (k_encode's
 // input, 16 bytes), so the first round reads it instead of a 128-byte h0 row.
@@ -340,230 +341,254 @@ __global__ void k_pack_input(int n, const double* __restrict__ r, const double* 
     xin[i] = make_float4(x0, feats[i], feats[n + i], feats[2 * n + i]);
 }
 
-// The first round's input state h0 = relu(W_in x + b_in), formed where the
-// round reads it (k_encode's arithmetic) instead of being written by a
-// separate kernel and read back: one lane's quarter-row (four features).
+// One row's state of the lane's eight features as FP32.  BF16 -> FP32 is
+// exact: the BF16 bits are the upper half of the FP32 word.
+__device__ __forceinline__ void unpack8(uint4 u, float (&f)[8]) {
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        f[2 * q] = __uint_as_float(w[q] << 16);
+        f[2 * q + 1] = __uint_as_float(w[q] & 0xffff0000u);
+    }
+}
+
+// The first round's state h0 = relu(W_in x + b_in), formed where the round
+// reads it (k_encode's arithmetic) instead of being written by a separate
+// kernel and read back: the lane's eight features.
 struct Encoder {
-    const float4* xin;
-    float w[4][4], b[4];
-    __device__ __forceinline__ void load(const float4* xin_, const float* P, int quarter) {
-        xin = xin_;
+    float w[8][4], b[8];
+    __device__ __forceinline__ void load(const float* P, int t) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int f = 4 * quarter + q;
-            b[q] = P[OFF_BIN + f];
+        for (int q = 0; q < 8; ++q) {
+            b[q] = P[OFF_BIN + 8 * t + q];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) w[q][c] = P[OFF_WIN + f * 4 + c];
+            for (int c = 0; c < 4; ++c) w[q][c] = P[OFF_WIN + (8 * t + q) * 4 + c];
         }
     }
-    __device__ __forceinline__ float4 h0(int j) const {
-        const float4 x = xin[j];
-        float o[4];
+    __device__ __forceinline__ void h0(float4 x, float (&f)[8]) const {
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-            o[q] = fmaxf(b[q] + w[q][0] * x.x + w[q][1] * x.y + w[q][2] * x.z + w[q][3] * x.w, 0.0f);
-        return make_float4(o[0], o[1], o[2], o[3]);
+        for (int q = 0; q < 8; ++q)
+            f[q] = fmaxf(b[q] + w[q][0] * x.x + w[q][1] * x.y + w[q][2] * x.z + w[q][3] * x.w, 0.0f);
     }
 };
 
-// Gather of one 16-cell tile: sH = h (FP32), sU = [h, a] (BF16), a_i = sum_j w_ij h_j.
-// Lanes 8q..8q+7 take cell 4 * pass + q, each lane one 16-byte quarter-row.
-// STAGED: the tile's couplings are in sIdx / sW (index k - seg_b); otherwise
-// they are read from global memory.  FIRST: h is the encoder's h0.
-// BF16 -> FP32 is exact: the BF16 bits are the upper half of the FP32 word.
-// Done with integer shifts and masks (the ALU), which measured faster here
-// than the conversion instructions.
-__device__ __forceinline__ float4 unpack_bf16x4(uint2 u) {
-    return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u),
-                       __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
-}
+// The couplings of one tile row: its range, and this lane's entry of the first four.
+struct RowCouplings {
+    int b, e, j;
+    float w;
+};
 
-template <bool STAGED, bool FIRST>
-__device__ __forceinline__ void gather_tile(int c0, int cells, int rb, int re, int seg_b, const int* sIdx,
-                                            const float* sW, const int* __restrict__ gco,
-                                            const float* __restrict__ gew, const __nv_bfloat16* __restrict__ h_in,
-                                            const Encoder& enc, float (*sH)[F], __nv_bfloat16 (*sU)[kUPad]) {
-    const int lane = threadIdx.x & 31;
-    // the state between rounds is BF16: a lane's quarter-row is 8 bytes
-    const uint2* h8 = reinterpret_cast<const uint2*>(h_in);
-    const int grp = lane >> 3, quarter = lane & 7;
-    // 32-bit row offsets (the binding keeps n * F / 4 below 2^31)
-    auto hrow = [&](int j) -> float4 {
-        if constexpr (FIRST) return enc.h0(j);
-        else return unpack_bf16x4(h8[j * (F / 4) + quarter]);
-    };
-    // the four passes unrolled: their neighbour rows are loaded together
-#pragma unroll
-    for (int pass = 0; pass < kTileCells / 4; ++pass) {
-        const int r = pass * 4 + grp;
-        const int b = __shfl_sync(0xffffffffu, rb, r), e = __shfl_sync(0xffffffffu, re, r);
-        float4 hv = make_float4(0.f, 0.f, 0.f, 0.f), av = make_float4(0.f, 0.f, 0.f, 0.f);
-        const int self = r < cells ? c0 + r : c0;
-        if (r < cells) hv = hrow(self);
-        // neighbours four at a time, the last group predicated (a tet cell has
-        // at most four): the padding terms read the cell's own row with weight 0
-        for (int k0 = b; k0 < e; k0 += 4) {
-            int j[4];
-            float w[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int k = k0 + u;
-                const bool ok = k < e;
-                j[u] = ok ? (STAGED ? sIdx[k - seg_b] : gco[k]) : self;
-                w[u] = ok ? (STAGED ? sW[k - seg_b] : gew[k]) : 0.0f;
-            }
-            float4 v[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) v[u] = hrow(j[u]);
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                av.x += w[u] * v[u].x; av.y += w[u] * v[u].y; av.z += w[u] * v[u].z; av.w += w[u] * v[u].w;
-            }
+__device__ __forceinline__ RowCouplings load_couplings(int cell, int n, int t, const int* __restrict__ gro,
+                                                       const int* __restrict__ gco, const float* __restrict__ gew) {
+    RowCouplings c{0, 0, cell < n ? cell : 0, 0.0f};
+    if (cell < n) {
+        c.b = gro[cell];
+        c.e = gro[cell + 1];
+        if (c.b + t < c.e) {
+            c.j = gco[c.b + t];
+            c.w = gew[c.b + t];
         }
-        *reinterpret_cast<float4*>(&sH[r][4 * quarter]) = hv;
-        uint2 hp, ap;
-        hp.x = pack_bf16(hv.x, hv.y); hp.y = pack_bf16(hv.z, hv.w);
-        ap.x = pack_bf16(av.x, av.y); ap.y = pack_bf16(av.z, av.w);
-        *reinterpret_cast<uint2*>(&sU[r][4 * quarter]) = hp;
-        *reinterpret_cast<uint2*>(&sU[r][F + 4 * quarter]) = ap;
     }
+    return c;
 }
 
 // One round.  FIRST: the input state is formed from r by the encoder (no h0
 // in memory).  LAST: the new state goes straight to the readout,
 // out_i = s (w_out . h_i + b_out) / a_ii, instead of to h_out.
 template <bool FIRST, bool LAST>
-__global__ void __launch_bounds__(kRoundThreads) k_round_gather_tc(
+__global__ void __launch_bounds__(kRoundThreads, FIRST ? 2 : 4) k_round_gather_tc(
     int n, const int* __restrict__ gro, const int* __restrict__ gco, const float* __restrict__ gew,
-    const __nv_bfloat16* __restrict__ h_in, __nv_bfloat16* __restrict__ h_out, const __nv_bfloat16* __restrict__ W1g,
-    const __nv_bfloat16* __restrict__ W2g, const float* __restrict__ Pr, const float* __restrict__ P,
-    const double* __restrict__ r, const double* __restrict__ rr, const float* __restrict__ feats,
-    const double* __restrict__ diag, double* __restrict__ yout) {
-    __shared__ __align__(16) __nv_bfloat16 sW1[F][kUPad];
-    __shared__ __align__(16) __nv_bfloat16 sW2[F][kW2Pad];
-    __shared__ __align__(16) __nv_bfloat16 sU[kRoundWarps][kTileCells][kUPad];
-    __shared__ __align__(16) float sH[kRoundWarps][kTileCells][F];
-    __shared__ int sIdx[kRoundWarps][kSegCap];
-    __shared__ float sW[kRoundWarps][kSegCap];
-    __shared__ float sb1[F], sb2[F];
-    for (int q = threadIdx.x; q < F * 2 * F; q += blockDim.x) sW1[q / (2 * F)][q % (2 * F)] = W1g[q];
-    for (int q = threadIdx.x; q < F * F; q += blockDim.x) sW2[q / F][q % F] = W2g[q];
-    if (threadIdx.x < F) {
-        sb1[threadIdx.x] = Pr[OFF_B1 + threadIdx.x];
-        sb2[threadIdx.x] = Pr[OFF_B2 + threadIdx.x];
-    }
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const float4* __restrict__ xin, const __nv_bfloat16* __restrict__ h_in, __nv_bfloat16* __restrict__ h_out,
+    const __nv_bfloat16* __restrict__ W1g, const __nv_bfloat16* __restrict__ W2g, const float* __restrict__ Pr,
+    const float* __restrict__ P, const double* __restrict__ rr, const double* __restrict__ diag,
+    double* __restrict__ yout) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    // B operands: k slots numbered as above for W1 (k blocks 0, 1: h; 2, 3: a);
+    // W2 takes layer 1's output columns in their natural order and gives output
+    // column 8 j + n as feature 8 (n / 2) + 2 j + n % 2
+    uint32_t w1[4][4][2], w2[2][4][2];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const __nv_bfloat16* row = W1g + (8 * j + g) * (2 * F) + (k & 2) * (F / 2) + 8 * t + 4 * (k & 1);
+            w1[k][j][0] = ld32(row);
+            w1[k][j][1] = ld32(row + 2);
+        }
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const __nv_bfloat16* row = W2g + (8 * (g >> 1) + 2 * j + (g & 1)) * F + 16 * k + 2 * t;
+            w2[k][j][0] = ld32(row);
+            w2[k][j][1] = ld32(row + 8);
+        }
     Encoder enc;
-    if constexpr (FIRST) enc.load(reinterpret_cast<const float4*>(feats), P, lane & 7);
-    // persistent: each warp walks tiles with the grid's stride, the weights
-    // staged once per block
-    for (int tile = blockIdx.x * kRoundWarps + warp; tile * kTileCells < n; tile += gridDim.x * kRoundWarps) {
-    const int c0 = tile * kTileCells;
-    const int cells = min(kTileCells, n - c0);
-    // tile segment of the coupling list
-    const int seg_b = gro[c0], seg_e = gro[c0 + cells];
-    const bool staged = seg_e - seg_b <= kSegCap;
-    if (staged)
-        for (int q = lane; q < seg_e - seg_b; q += 32) {
-            sIdx[warp][q] = gco[seg_b + q];
-            sW[warp][q] = gew[seg_b + q];
+    if constexpr (FIRST) enc.load(P, t);
+    const double scale = LAST ? sqrt(*rr / n) : 0.0;
+    const uint4* h16 = reinterpret_cast<const uint4*>(h_in);
+    const int warps = gridDim.x * (kRoundThreads / 32);
+    int tile = blockIdx.x * (kRoundThreads / 32) + (threadIdx.x >> 5);
+    if (tile * kTileCells >= n) return;
+    RowCouplings cur[2];
+#pragma unroll
+    for (int p = 0; p < 2; ++p) cur[p] = load_couplings(tile * kTileCells + g + 8 * p, n, t, gro, gco, gew);
+    for (; tile * kTileCells < n; tile += warps) {
+        const int c0 = tile * kTileCells;
+        float hv[2][8], av[2][8];
+        uint32_t ah[2][4];
+        // the first four neighbours of both rows, all loads in flight together
+        if constexpr (FIRST) {
+            float4 xo[2], xn[2][4];
+            float w[2][4];
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                const int cell = min(c0 + g + 8 * p, n - 1);
+                xo[p] = xin[cell];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    xn[p][u] = xin[__shfl_sync(0xffffffffu, cur[p].j, u, 4)];
+                    w[p][u] = __shfl_sync(0xffffffffu, cur[p].w, u, 4);
+                }
+            }
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                enc.h0(xo[p], hv[p]);
+#pragma unroll
+                for (int q = 0; q < 8; ++q) av[p][q] = 0.0f;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    float v[8];
+                    enc.h0(xn[p][u], v);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) av[p][q] += w[p][u] * v[q];
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) ah[p][q] = pack_bf16(hv[p][2 * q], hv[p][2 * q + 1]);
+            }
+        } else {
+            uint4 own[2], nb[2][4];
+            float w[2][4];
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                const int cell = min(c0 + g + 8 * p, n - 1);
+                own[p] = h16[cell * (F / 8) + t];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    nb[p][u] = h16[__shfl_sync(0xffffffffu, cur[p].j, u, 4) * (F / 8) + t];
+                    w[p][u] = __shfl_sync(0xffffffffu, cur[p].w, u, 4);
+                }
+            }
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                unpack8(own[p], hv[p]);
+                ah[p][0] = own[p].x; ah[p][1] = own[p].y; ah[p][2] = own[p].z; ah[p][3] = own[p].w;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) av[p][q] = 0.0f;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    float v[8];
+                    unpack8(nb[p][u], v);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) av[p][q] += w[p][u] * v[q];
+                }
+            }
         }
-    int rb = 0, re = 0;   // lanes 0..15: row range of cell c0 + lane
-    if (lane < cells) {
-        rb = gro[c0 + lane];
-        re = gro[c0 + lane + 1];
-    }
-    __syncwarp();
-    if (staged)
-        gather_tile<true, FIRST>(c0, cells, rb, re, seg_b, sIdx[warp], sW[warp], gco, gew, h_in, enc, sH[warp],
-                                 sU[warp]);
-    else
-        gather_tile<false, FIRST>(c0, cells, rb, re, seg_b, sIdx[warp], sW[warp], gco, gew, h_in, enc, sH[warp],
-                                  sU[warp]);
-    __syncwarp();
-    const int g = lane >> 2, t = lane & 3;
-    float acc[4][4];
+        // rows of more than four neighbours
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        acc[j][0] = sb1[8 * j + 2 * t];
-        acc[j][1] = sb1[8 * j + 2 * t + 1];
-        acc[j][2] = sb1[8 * j + 2 * t];
-        acc[j][3] = sb1[8 * j + 2 * t + 1];
-    }
+        for (int p = 0; p < 2; ++p)
+            for (int k0 = cur[p].b + 4; __any_sync(0xffffffffu, k0 < cur[p].e); k0 += 4) {
+                const int self = min(c0 + g + 8 * p, n - 1);
+                const int j = k0 + t < cur[p].e ? gco[k0 + t] : self;
+                const float wj = k0 + t < cur[p].e ? gew[k0 + t] : 0.0f;
 #pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-        const uint32_t a0 = ld32(&sU[warp][g][16 * kk + 2 * t]);
-        const uint32_t a1 = ld32(&sU[warp][g + 8][16 * kk + 2 * t]);
-        const uint32_t a2 = ld32(&sU[warp][g][16 * kk + 2 * t + 8]);
-        const uint32_t a3 = ld32(&sU[warp][g + 8][16 * kk + 2 * t + 8]);
+                for (int u = 0; u < 4; ++u) {
+                    const int ju = __shfl_sync(0xffffffffu, j, u, 4);
+                    const float wu = __shfl_sync(0xffffffffu, wj, u, 4);
+                    float v[8];
+                    if constexpr (FIRST) enc.h0(xin[ju], v);
+                    else unpack8(h16[ju * (F / 8) + t], v);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) av[p][q] += wu * v[q];
+                }
+            }
+        // the next tile's couplings, in flight during the products
+        if ((tile + warps) * kTileCells < n) {
+#pragma unroll
+            for (int p = 0; p < 2; ++p)
+                cur[p] = load_couplings((tile + warps) * kTileCells + g + 8 * p, n, t, gro, gco, gew);
+        }
+        float acc[4][4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const uint32_t b0 = ld32(&sW1[8 * j + g][16 * kk + 2 * t]);
-            const uint32_t b1 = ld32(&sW1[8 * j + g][16 * kk + 2 * t + 8]);
-            mma_bf16(acc[j], a0, a1, a2, a3, b0, b1);
+            const float2 b1 = *reinterpret_cast<const float2*>(Pr + OFF_B1 + 8 * j + 2 * t);
+            acc[j][0] = acc[j][2] = b1.x;
+            acc[j][1] = acc[j][3] = b1.y;
         }
-    }
-    uint32_t A2[2][4];
 #pragma unroll
-    for (int kk = 0; kk < 2; ++kk) {
-        A2[kk][0] = pack_bf16(fmaxf(acc[2 * kk][0], 0.f), fmaxf(acc[2 * kk][1], 0.f));
-        A2[kk][1] = pack_bf16(fmaxf(acc[2 * kk][2], 0.f), fmaxf(acc[2 * kk][3], 0.f));
-        A2[kk][2] = pack_bf16(fmaxf(acc[2 * kk + 1][0], 0.f), fmaxf(acc[2 * kk + 1][1], 0.f));
-        A2[kk][3] = pack_bf16(fmaxf(acc[2 * kk + 1][2], 0.f), fmaxf(acc[2 * kk + 1][3], 0.f));
-    }
-    float out[4][4];
+        for (int k = 0; k < 2; ++k)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int col = 8 * j + 2 * t;
-        out[j][0] = sb2[col] + sH[warp][g][col];
-        out[j][1] = sb2[col + 1] + sH[warp][g][col + 1];
-        out[j][2] = sb2[col] + sH[warp][g + 8][col];
-        out[j][3] = sb2[col + 1] + sH[warp][g + 8][col + 1];
-    }
+            for (int j = 0; j < 4; ++j)
+                mma_bf16(acc[j], ah[0][2 * k], ah[1][2 * k], ah[0][2 * k + 1], ah[1][2 * k + 1], w1[k][j][0],
+                         w1[k][j][1]);
 #pragma unroll
-    for (int kk = 0; kk < 2; ++kk) {
+        for (int k = 0; k < 2; ++k) {
+            const uint32_t a0 = pack_bf16(av[0][4 * k], av[0][4 * k + 1]);
+            const uint32_t a1 = pack_bf16(av[1][4 * k], av[1][4 * k + 1]);
+            const uint32_t a2 = pack_bf16(av[0][4 * k + 2], av[0][4 * k + 3]);
+            const uint32_t a3 = pack_bf16(av[1][4 * k + 2], av[1][4 * k + 3]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) mma_bf16(acc[j], a0, a1, a2, a3, w1[2 + k][j][0], w1[2 + k][j][1]);
+        }
+        float out[4][4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const uint32_t b0 = ld32(&sW2[8 * j + g][16 * kk + 2 * t]);
-            const uint32_t b1 = ld32(&sW2[8 * j + g][16 * kk + 2 * t + 8]);
-            mma_bf16(out[j], A2[kk][0], A2[kk][1], A2[kk][2], A2[kk][3], b0, b1);
+            const float2 b2 = *reinterpret_cast<const float2*>(Pr + OFF_B2 + 8 * t + 2 * j);
+            out[j][0] = b2.x + hv[0][2 * j];
+            out[j][1] = b2.y + hv[0][2 * j + 1];
+            out[j][2] = b2.x + hv[1][2 * j];
+            out[j][3] = b2.y + hv[1][2 * j + 1];
         }
-    }
-    const int rowa = g, rowb = g + 8;
-    if constexpr (LAST) {
-        // readout: row sums over this lane's columns, then across the 4 lanes of the row
-        float ya = 0.0f, yb = 0.0f;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int col = 8 * j + 2 * t;
-            const float w0 = P[OFF_WOUT + col], w1 = P[OFF_WOUT + col + 1];
-            ya += w0 * out[j][0] + w1 * out[j][1];
-            yb += w0 * out[j][2] + w1 * out[j][3];
-        }
-        ya += __shfl_xor_sync(0xffffffffu, ya, 1);
-        ya += __shfl_xor_sync(0xffffffffu, ya, 2);
-        yb += __shfl_xor_sync(0xffffffffu, yb, 1);
-        yb += __shfl_xor_sync(0xffffffffu, yb, 2);
-        if (t == 0) {
-            const double s = sqrt(*rr / n);
-            const float bo = P[OFF_BOUT];
-            if (rowa < cells) yout[c0 + rowa] = s * static_cast<double>(ya + bo) / diag[c0 + rowa];
-            if (rowb < cells) yout[c0 + rowb] = s * static_cast<double>(yb + bo) / diag[c0 + rowb];
-        }
-    } else {
+        for (int k = 0; k < 2; ++k) {
+            const uint32_t a0 = pack_bf16(fmaxf(acc[2 * k][0], 0.f), fmaxf(acc[2 * k][1], 0.f));
+            const uint32_t a1 = pack_bf16(fmaxf(acc[2 * k][2], 0.f), fmaxf(acc[2 * k][3], 0.f));
+            const uint32_t a2 = pack_bf16(fmaxf(acc[2 * k + 1][0], 0.f), fmaxf(acc[2 * k + 1][1], 0.f));
+            const uint32_t a3 = pack_bf16(fmaxf(acc[2 * k + 1][2], 0.f), fmaxf(acc[2 * k + 1][3], 0.f));
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int col = 8 * j + 2 * t;
-            if (rowa < cells)
-                *reinterpret_cast<uint32_t*>(&h_out[static_cast<size_t>(c0 + rowa) * F + col]) =
-                    pack_bf16(out[j][0], out[j][1]);
-            if (rowb < cells)
-                *reinterpret_cast<uint32_t*>(&h_out[static_cast<size_t>(c0 + rowb) * F + col]) =
-                    pack_bf16(out[j][2], out[j][3]);
+            for (int j = 0; j < 4; ++j) mma_bf16(out[j], a0, a1, a2, a3, w2[k][j][0], w2[k][j][1]);
         }
-    }
-    __syncwarp();   // the warp's sU / sH are rewritten by its next tile
+        if constexpr (LAST) {
+            // readout: row sums over this lane's features, then across the 4 lanes of the row
+            float ya = 0.0f, yb = 0.0f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float wo0 = P[OFF_WOUT + 8 * t + 2 * j], wo1 = P[OFF_WOUT + 8 * t + 2 * j + 1];
+                ya += wo0 * out[j][0] + wo1 * out[j][1];
+                yb += wo0 * out[j][2] + wo1 * out[j][3];
+            }
+            ya += __shfl_xor_sync(0xffffffffu, ya, 1);
+            ya += __shfl_xor_sync(0xffffffffu, ya, 2);
+            yb += __shfl_xor_sync(0xffffffffu, yb, 1);
+            yb += __shfl_xor_sync(0xffffffffu, yb, 2);
+            if (t == 0) {
+                const float bo = P[OFF_BOUT];
+                const int ra = c0 + g, rb = c0 + g + 8;
+                if (ra < n) yout[ra] = scale * static_cast<double>(ya + bo) / diag[ra];
+                if (rb < n) yout[rb] = scale * static_cast<double>(yb + bo) / diag[rb];
+            }
+        } else {
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                const int row = c0 + g + 8 * p;
+                if (row < n)
+                    reinterpret_cast<uint4*>(h_out)[row * (F / 8) + t] =
+                        make_uint4(pack_bf16(out[0][2 * p], out[0][2 * p + 1]),
+                                   pack_bf16(out[1][2 * p], out[1][2 * p + 1]),
+                                   pack_bf16(out[2][2 * p], out[2][2 * p + 1]),
+                                   pack_bf16(out[3][2 * p], out[3][2 * p + 1]));
+            }
+        }
     }
 }
 
@@ -1007,16 +1032,13 @@ void infer(cfdxg_context* ctx, cfdxg_mpnn* net, const double* r, double* out) {
                      in_bytes + out_bytes + 4.0 * (n + 1) + 8.0 * static_cast<double>(net->gco.size()));
         auto kern = first ? k_round_gather_tc<true, false>
                           : (last ? k_round_gather_tc<false, true> : k_round_gather_tc<false, false>);
-        // persistent grid of five blocks per SM (the shared-memory limit) for
-        // the middle and last rounds: 166 / 171 instead of 210 / 220 us at
-        // 64^3.  The first round, which forms h0 per neighbour, measured
-        // slower that way (277 vs 243 us) and takes one tile per warp.
-        const int all = (tiles + kRoundWarps - 1) / kRoundWarps;
-        const int grid = first ? all : std::min(all, 5 * ctx->sm_count);
-        kern<<<grid, kRoundThreads, 0, s>>>(
-            n, net->gro.get(), net->gco.get(), net->gew.get(), hin, hout, w, w + 2 * F * F,
-            net->params.get() + ROUND0 + k * ROUND_SIZE, net->params.get(), r, rr,
-            first ? reinterpret_cast<const float*>(xin) : nullptr, net->diag.get(), out);
+        // one resident wave (two blocks per SM in the first round, whose lanes
+        // hold the encoder's weights too, four of 128 registers in the others)
+        const int all = (tiles + kRoundThreads / 32 - 1) / (kRoundThreads / 32);
+        const int grid = std::min(all, (first ? 2 : 4) * ctx->sm_count);
+        kern<<<grid, kRoundThreads, 0, s>>>(n, net->gro.get(), net->gco.get(), net->gew.get(), xin, hin, hout, w,
+                                            w + 2 * F * F, net->params.get() + ROUND0 + k * ROUND_SIZE,
+                                            net->params.get(), rr, net->diag.get(), out);
         check_launch(ctx);
         std::swap(hin, hout);
     }

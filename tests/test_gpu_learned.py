@@ -101,6 +101,27 @@ def test_tensor_core_inference_matches_oracle(bound):
     assert np.allclose(net.apply(2.0 * r), 2.0 * y, rtol=1e-5, atol=1e-12 * np.abs(y).max())
 
 
+@pytest.mark.parametrize("kind", ["tet1", "tet3", "tet7", "hex4", "layer"])
+def test_inference_tiles_and_neighbour_counts(ctx, kind):
+    """Fewer cells than a 16-cell tile, remainder tiles, more than four
+    neighbours per cell; the same bound as above (BF16 operands and state)."""
+    if kind.startswith("tet"):
+        m = cases.simple_mesh(int(kind[3:]))
+    else:
+        m = cg.hex_case(4, 3, 5) if kind == "hex4" else cg.boundary_layer_case(9, 13, 7)
+    mesh = cg.Mesh(ctx, m)
+    g = mesh.geometry()
+    U, rAU, aP, p, fixed, value = cases.simple_fields(m, g["cell_centres"])
+    A, b, phi, grad = cg.assemble_pressure_correction(mesh, U, rAU, p, 1.0, fixed, value)
+    G = mo.Graph(*A.to_csr(), g["cell_volumes"], aP)
+    net = cg.LearnedPreconditioner(ctx, seed=3)
+    net.bind(mesh, A, aP)
+    net.set_parameters(mo.init_params(5).astype(np.float32))
+    r = np.random.default_rng(4).standard_normal(G.n)
+    y, y_ref = net.apply(r), mo.forward(net.parameters().astype(np.float64), G, r)
+    assert np.linalg.norm(y - y_ref) <= 3e-2 * np.linalg.norm(y_ref)
+
+
 def test_training_reduces_loss_and_weights_roundtrip(bound, tmp_path):
     G, net = bound["G"], bound["net"]
     R, E = _pairs(G, 4, seed=1)

@@ -664,3 +664,24 @@ def test_own_diagonal_cg_refuses_negative_curvature(ctx):
     A = cg.SparseMatrix.from_csr(ctx, ro, co, np.array([1.0, 2.0, 2.0, 1.0]))
     x, rep = cg.solve_linear_system(A, np.array([1.0, -1.0]), krylov="cg", preconditioner="own_diagonal")
     assert rep["status_name"] == "not_applicable" and np.array_equal(x, np.zeros(2))
+
+
+@pytest.mark.parametrize("n_patches", [1, 32, 33, 40])
+def test_patch_tables_in_the_launch_and_on_the_device(ctx, oracle, n_patches):
+    """Boundary faces spread over n_patches patches, every third fixed: up to
+    32 patches the table travels in the launch, beyond in device memory."""
+    m = cases.simple_mesh(3)
+    rng = np.random.default_rng(n_patches)
+    bnd = m.neighbour < 0
+    m.patch_of_face[bnd] = rng.integers(0, n_patches, bnd.sum()).astype(np.int32)
+    m.patch_types = np.zeros(n_patches, np.int32)
+    fixed = (np.arange(n_patches) % 3 == 0).astype(np.int32)
+    value = rng.standard_normal(n_patches)
+    mesh = cg.Mesh(ctx, m)
+    U, rAU, aP, _, _, _ = cases.simple_fields(m, mesh.geometry()["cell_centres"])
+    p = rng.standard_normal(m.n_cells)
+    A, b, phi, grad = cg.assemble_pressure_correction(mesh, U, rAU, p, 1.0, fixed, value)
+    ref = oracle.simple_assemble(m, U, rAU, p, 1.0, fixed, value)
+    assert np.array_equal(A.to_csr()[2], ref["values"]) and np.array_equal(b, ref["b"])
+    assert np.array_equal(cg.make_rhie_chow_mass_flux(mesh, U, rAU, p, 1.0, fixed, value),
+                          oracle.rhie_chow_flux(m, U, rAU, p, 1.0, fixed, value))
