@@ -18,10 +18,9 @@
 // left transposed for the next kernel) and the rank-64 update of the lower
 // tiles, whose first block also inverts the next pivot block, so that the
 // serial part hides behind the update.  Bound by FP64 multiply-adds (n^3 of
-// them in all) on large levels and by the serial pivots (47 us per block
-// column) on small ones.  3,429 rows: 4.4 ms, against 10.5 ms by cuSOLVER's
-// potrf and potri, whose triangular inverse and product run in many small
-// kernels.
+// them in all) on large levels and by the serial pivots on small ones.  3,429
+// rows: 3.6 ms, against 10.5 ms by cuSOLVER's potrf and potri, whose triangular
+// inverse and product run in many small kernels.
 #include "dense.h"
 
 #include <cmath>
@@ -59,43 +58,49 @@ __device__ __forceinline__ void tile_product(const double* a, int lda, const dou
 
 // Inverts the 64 x 64 symmetric block held 4 x 4 per thread (rows part(ty, .),
 // columns part(tx, .)) by 64 scalar sweeps; *info = 1 when a pivot is not
-// positive and finite.  rowbuf, colbuf: 2 x 64 doubles of shared memory.
+// positive and finite.  The pivots are taken by their place in the threads'
+// parts (any order of a positive definite block will do), so that the pivot
+// row and column sit in fixed registers of the threads that hold them: with
+// the place known only at run time, selecting it cost more instructions than
+// the sweep and the block took 47 us.  rowbuf, colbuf: 2 x 64 doubles of shared
+// memory.
 __device__ void invert_block(double (&v)[4][4], int ty, int tx, double* rowbuf, double* colbuf, int* info) {
-    for (int p = 0; p < kB; ++p) {
-        double* rb = rowbuf + (p & 1) * kB;
-        double* cb = colbuf + (p & 1) * kB;
-        const int pq = (p & 31) >> 1, pu = ((p >> 5) << 1) | (p & 1);   // p = part(pq, pu)
-        if (ty == pq) {
+#pragma unroll
+    for (int pu = 0; pu < 4; ++pu) {
+#pragma unroll 1
+        for (int pq = 0; pq < 16; ++pq) {
+            const int p = part(pq, pu);
+            double* rb = rowbuf + (pq & 1) * kB;
+            double* cb = colbuf + (pq & 1) * kB;
+            if (ty == pq) {
+                *reinterpret_cast<double2*>(rb + 2 * tx) = make_double2(v[pu][0], v[pu][1]);
+                *reinterpret_cast<double2*>(rb + 32 + 2 * tx) = make_double2(v[pu][2], v[pu][3]);
+            }
+            if (tx == pq) {
+                *reinterpret_cast<double2*>(cb + 2 * ty) = make_double2(v[0][pu], v[1][pu]);
+                *reinterpret_cast<double2*>(cb + 32 + 2 * ty) = make_double2(v[2][pu], v[3][pu]);
+            }
+            __syncthreads();
+            const double pivot = rb[p];
+            if (!(pivot > 0.0) || !isfinite(pivot)) *info = 1;
+            const double inv = 1.0 / pivot;
+            double r[4], c[4];
+            load4(rb, tx, r);
+            load4(cb, ty, c);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) r[j] *= inv;
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-                if (i == pu)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) rb[part(tx, j)] = v[i][j];
-        }
-        if (tx == pq) {
+                for (int j = 0; j < 4; ++j) v[i][j] -= c[i] * r[j];
+            if (ty == pq) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (j == pu)
+                for (int j = 0; j < 4; ++j) v[pu][j] = r[j];
+            }
+            if (tx == pq) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) cb[part(ty, i)] = v[i][j];
-        }
-        __syncthreads();
-        const double pivot = rb[p];
-        if (!(pivot > 0.0) || !isfinite(pivot)) *info = 1;
-        const double inv = 1.0 / pivot;
-        double r[4], c[4];
-        load4(rb, tx, r);
-        load4(cb, ty, c);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const bool prow = ty == pq && i == pu;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const bool pcol = tx == pq && j == pu;
-                const double rj = inv * r[j];
-                if (prow) v[i][j] = pcol ? inv : rj;
-                else if (pcol) v[i][j] = -c[i] * inv;
-                else v[i][j] -= c[i] * rj;
+                for (int i = 0; i < 4; ++i) v[i][pu] = -c[i] * inv;
+                if (ty == pq) v[pu][pu] = inv;
             }
         }
     }
