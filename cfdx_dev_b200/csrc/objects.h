@@ -102,7 +102,7 @@ struct cfdxg_mesh {
     // slot (cell-face order) the face id, with bit 31 set where the cell is
     // the face's neighbour, and the other cell (-1 on the boundary); the Gauss
     // gradient's interpolation weight of the cell's side; per face the
-    // corrector's geometric terms d, e, Sf . e (5 x n_faces, SoA)
+    // corrector's geometric terms d, e (4 x n_faces, SoA)
     cfdxg::DevBuf<int2> slot_rec;
     cfdxg::DevBuf<double> slot_w, face_geo;
     // per-call boundary table and gradient scratch, kept so the face-loop entry
