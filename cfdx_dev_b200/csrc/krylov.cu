@@ -243,7 +243,7 @@ __global__ void k_multi_axpy(int n, const double* __restrict__ V, int i0, int c,
     }
 }
 
-// ---- fused classical Gram-Schmidt passes (the CGS2 option, at most kChunk
+// ---- fused classical Gram-Schmidt passes (the CGS2 option, at most kFused
 // basis vectors): three passes over the basis per Arnoldi step instead of
 // four, and the two norms of w taken inside them (plain sums of squares: this
 // option is the library's own orthogonalisation, not the reference's MGS2).
@@ -253,6 +253,11 @@ __global__ void k_multi_axpy(int n, const double* __restrict__ V, int i0, int c,
 // per warp by a fixed butterfly, per block in warp order, and over the
 // blocks by one warp per output in a fixed lane/butterfly order.
 constexpr int kGsWarps = kT / 32;
+// Basis vectors the fused passes are instantiated for: a whole cycle of the
+// usual restarts (30).  Beyond, chunks of kChunk vectors per launch.  (With the
+// fused passes ending at 16 vectors, steps 17 and 18 of a 298,000-cell boundary
+// layer's solve took 140 us each in the chunked kernels.)
+constexpr int kFused = 32;
 
 // out[q] = grid sum of acc[q] for q < C; with EXTRA also out[C] = grid sum of extra.
 template <int C, bool EXTRA>
@@ -384,7 +389,7 @@ int resident_per_sm() {
     return per_sm;
 }
 
-// Calls go(std::integral_constant<int, C>) for the basis count c in 1..kChunk.
+// Calls go(std::integral_constant<int, C>) for the basis count c in 1..kFused.
 template <class Go>
 void with_basis_count(int c, Go&& go) {
     switch (c) {
@@ -392,6 +397,9 @@ void with_basis_count(int c, Go&& go) {
         CFDXG_GS_CASE(1) CFDXG_GS_CASE(2) CFDXG_GS_CASE(3) CFDXG_GS_CASE(4) CFDXG_GS_CASE(5) CFDXG_GS_CASE(6)
         CFDXG_GS_CASE(7) CFDXG_GS_CASE(8) CFDXG_GS_CASE(9) CFDXG_GS_CASE(10) CFDXG_GS_CASE(11)
         CFDXG_GS_CASE(12) CFDXG_GS_CASE(13) CFDXG_GS_CASE(14) CFDXG_GS_CASE(15) CFDXG_GS_CASE(16)
+        CFDXG_GS_CASE(17) CFDXG_GS_CASE(18) CFDXG_GS_CASE(19) CFDXG_GS_CASE(20) CFDXG_GS_CASE(21) CFDXG_GS_CASE(22)
+        CFDXG_GS_CASE(23) CFDXG_GS_CASE(24) CFDXG_GS_CASE(25) CFDXG_GS_CASE(26) CFDXG_GS_CASE(27) CFDXG_GS_CASE(28)
+        CFDXG_GS_CASE(29) CFDXG_GS_CASE(30) CFDXG_GS_CASE(31) CFDXG_GS_CASE(32)
 #undef CFDXG_GS_CASE
         default: throw Error(CFDXG_ERR_INVALID_ARGUMENT, "Gram-Schmidt basis count out of range");
     }
@@ -544,7 +552,7 @@ struct Workspace {
     int m = 0;
     DevBuf<double> V, Z, w, r, ax, best, trial, tmp;
     DevBuf<double> ns1, ns2, ns_partials;   // the projected operator's scratch
-    DevBuf<double> mpartial;   // (kChunk + 1) x kWideBlocks partial sums of the multi-dot
+    DevBuf<double> mpartial;   // (kFused + 1) x kWideBlocks partial sums of the multi-dot
     std::unique_ptr<StepMirror> mirror;
 };
 
@@ -562,7 +570,7 @@ Workspace& workspace(cfdxg_context* ctx, int64_t n, int m) {
         ws->trial.resize(n); ws->tmp.resize(n);
         ws->ns1.resize(n); ws->ns2.resize(n);
         ws->ns_partials.resize(kNsMaxBlocks);
-        ws->mpartial.resize(static_cast<size_t>(kChunk + 1) * kWideBlocks);
+        ws->mpartial.resize(static_cast<size_t>(kFused + 1) * kWideBlocks);
         ws->n = n;
         ws->m = mm;
     }
@@ -653,7 +661,7 @@ public:
         }
     }
     // Two passes of classical Gram-Schmidt of w against v_0..v_{count-1}
-    // (count <= kChunk) in three passes over the basis: h1 = V^T w (with the
+    // (count <= kFused) in three passes over the basis: h1 = V^T w (with the
     // action norm), w -= V h1 fused with h2 = V^T w, w -= V h2 fused with
     // ||w||.  Fills slots kH1.., kH2.., kAction and kHnext.
     // One resident wave of each pass (a fixed partition for a given count and
@@ -1243,7 +1251,7 @@ KrylovResult gmres_solve(cfdxg_context* ctx, const cfdxg_matrix* A, const double
             E.op(z(jj), ws->w.get());
             double* w = ws->w.get();
             int action_sq = -1;
-            if (controls.classical_gram_schmidt && jj + 1 <= kChunk) {
+            if (controls.classical_gram_schmidt && jj + 1 <= kFused) {
                 // classical Gram-Schmidt twice in three fused passes; the
                 // squared action norm comes from the first (slot kH1 + jj + 1)
                 E.gram_schmidt_cgs2_fused(V, jj + 1, w, ws->mpartial.get());
