@@ -13,8 +13,8 @@
 // memory, with deterministic weight-gradient reductions: each thread of a
 // block owns its gradient entries over a fixed set of tiles, and the blocks
 // are combined in a fixed order at the end.
-// Inference runs each round as one fused kernel: the neighbour gather builds
-// [h, a] in shared memory as BF16 and both MLP layers run on the tensor cores
+// Inference runs each round as one fused kernel: the neighbour gather leaves
+// [h, a] in the MMA's operand registers and both MLP layers run on the tensor cores
 // (mma.sync m16n8k16, BF16 operands, FP32 accumulation); the state h is
 // stored as BF16 between rounds and carried in FP32 within one.
 // The encoder is folded into the first round (h0 formed from r where it is
