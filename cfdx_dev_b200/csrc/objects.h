@@ -91,6 +91,7 @@ struct cfdxg_mesh {
     int64_t n_points = 0, n_faces = 0, n_cells = 0, n_internal = 0;
     int32_t n_patches = 0;
     int max_cell_faces = 0;
+    int uniform_faces = 0;   // faces of every cell, 0 when cells differ
     cfdxg::DevBuf<double> px, py, pz;
     cfdxg::DevBuf<int> face_off, face_vert, owner, neigh, cell_off, cell_face, cell_sorted,
         patch_of_face, patch_type;
