@@ -98,6 +98,48 @@ def test_pressure_assembly_other_cells_bit_exact(ctx, oracle, kind):
     assert np.array_equal(grad, r["grad_p"])
 
 
+def _union(meshes):
+    """Disjoint meshes as one (points, faces, cells and patches numbered on)."""
+    out = {k: [] for k in ("px", "py", "pz", "face_offsets", "face_vertices", "owner", "neighbour", "cell_offsets",
+                           "cell_faces", "patch_of_face", "patch_types")}
+    points = faces = cells = patches = verts = slots = 0
+    for m in meshes:
+        for k in ("px", "py", "pz", "patch_types"):
+            out[k].append(getattr(m, k))
+        first = 0 if not out["owner"] else 1
+        out["face_offsets"].append(m.face_offsets[first:] + verts)
+        out["cell_offsets"].append(m.cell_offsets[first:] + slots)
+        out["face_vertices"].append(m.face_vertices + points)
+        out["cell_faces"].append(m.cell_faces + faces)
+        out["owner"].append(m.owner + cells)
+        out["neighbour"].append(np.where(m.neighbour >= 0, m.neighbour + cells, m.neighbour))
+        out["patch_of_face"].append(np.where(m.patch_of_face >= 0, m.patch_of_face + patches, m.patch_of_face))
+        points, faces, cells = points + m.n_points, faces + m.n_faces, cells + m.n_cells
+        patches, verts, slots = patches + m.patch_types.size, verts + m.face_vertices.size, slots + m.cell_faces.size
+    return cg.HostMesh(**{k: np.concatenate(v).astype(getattr(meshes[0], k).dtype) for k, v in out.items()})
+
+
+@pytest.mark.parametrize("kinds", ["t", "h", "tp", "ph", "tph"])
+def test_face_loop_on_uniform_and_mixed_meshes_bit_exact(ctx, oracle, kinds):
+    """Every cell of four or of six faces (the forms whose slots need no look-up),
+    and cells of four, five and six faces in one mesh."""
+    make = {"t": lambda: cases.simple_mesh(1), "h": lambda: cg.boundary_layer_case(3, 2, 2),
+            "p": lambda: cases.prism_case(3, 2, 2)}
+    m = _union([make[k]() for k in kinds])
+    mesh = cg.Mesh(ctx, m)
+    g = mesh.geometry()
+    U, rAU, aP, p, fixed, value = cases.simple_fields(m, g["cell_centres"])
+    cc = g["cell_centres"].reshape(3, -1)
+    p1 = np.cos(2 * cc[0]) + cc[1] * cc[2]
+    value[0] = -0.5
+    A, b, phi, grad = cg.assemble_pressure_correction(mesh, U, rAU, p1, 1.1, fixed, value)
+    r = oracle.simple_assemble(m, U, rAU, p1, 1.1, fixed, value)
+    ro, co, va = A.to_csr()
+    assert np.array_equal(ro, r["row_offsets"]) and np.array_equal(co, r["columns"])
+    assert np.array_equal(va, r["values"]) and np.array_equal(b, r["b"])
+    assert np.array_equal(phi, r["phiHbyA"]) and np.array_equal(grad, r["grad_p"])
+
+
 def test_prism_pressure_solve_matches_oracle(ctx, oracle):
     # five-face cells end to end: the device setup equals the host setup, the
     # reference-order cycle is bit-identical to the oracle's, and the solve
