@@ -19,7 +19,7 @@
 // tiles, whose first block also inverts the next pivot block, so that the
 // serial part hides behind the update.  Bound by FP64 multiply-adds (n^3 of
 // them in all) on large levels and by the serial pivots on small ones.  3,429
-// rows: 3.6 ms, against 10.5 ms by cuSOLVER's potrf and potri, whose triangular
+// rows: 3.2 ms, against 10.5 ms by cuSOLVER's potrf and potri, whose triangular
 // inverse and product run in many small kernels.
 #include "dense.h"
 
@@ -167,14 +167,30 @@ __global__ void __launch_bounds__(kThreads) k_spd_panel(double* a, int ld, int k
     }
 }
 
+// d += a b on the FP64 tensor cores: a 8 x 4 (lane: row lane / 4, column lane
+// % 4), b 4 x 8 (row lane % 4, column lane / 4), d 8 x 8 (row lane / 4, columns
+// 2 (lane % 4) and the next).  FP64 multiply-adds throughout.
+__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(d[0]), "+d"(d[1])
+        : "d"(a), "d"(b));
+}
+
 // A_IJ -= W_I P_J^T for the lower tiles outside row and column k.  Block 0 takes
 // the next pivot tile and inverts it into d.
-__global__ void __launch_bounds__(kThreads) k_spd_update(double* a, int ld, int tiles, int k,
-                                                         const double* pt, const double* wt, double* d, int* info) {
+//
+// A warp takes 32 x 16 of the tile as 4 x 2 tensor products over 16 steps of
+// four k: six shared reads (two wavefronts each, kUpdateLd spreading the four k
+// over the banks) for 2,048 multiply-adds.  With 4 x 4 register tiles a thread's
+// shared reads took as long as its multiply-adds: 63 us a launch at 3,429 rows
+// against 43, of which block 0's serial pivots are most.
+constexpr int kUpdateLd = kB + 4;
+__global__ void __launch_bounds__(kThreads, 3) k_spd_update(double* a, int ld, int tiles, int k,
+                                                            const double* pt, const double* wt, double* d, int* info) {
     pdl_entry();
     extern __shared__ __align__(16) double smem[];
-    double* sw = smem;               // [k][row]
-    double* sp = smem + kB * kB;     // [k][column]
+    double* sw = smem;                     // [k][row]
+    double* sp = smem + kB * kUpdateLd;    // [k][column]
     const int count = (tiles - 1) * tiles / 2;   // lower tiles of the other tiles - 1 block rows
     // the next pivot tile (k + 1, k + 1) is lower tile (k, k) once row k is left out
     const int next = k + 1 < tiles ? k * (k + 1) / 2 + k : -1;
@@ -186,38 +202,55 @@ __global__ void __launch_bounds__(kThreads) k_spd_update(double* a, int ld, int 
     int J = t - I * (I + 1) / 2;
     if (I >= k) ++I;
     if (J >= k) ++J;
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
     for (int q = threadIdx.x; q < kB * kB / 2; q += kThreads) {
         const int r = q / (kB / 2), c = 2 * (q % (kB / 2));
-        *reinterpret_cast<double2*>(sw + r * kB + c) =
+        *reinterpret_cast<double2*>(sw + r * kUpdateLd + c) =
             *reinterpret_cast<const double2*>(wt + static_cast<size_t>(r) * ld + I * kB + c);
-        *reinterpret_cast<double2*>(sp + r * kB + c) =
+        *reinterpret_cast<double2*>(sp + r * kUpdateLd + c) =
             *reinterpret_cast<const double2*>(pt + static_cast<size_t>(r) * ld + J * kB + c);
     }
-    double v[4][4];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, m = lane & 3;
+    const int row0 = (warp & 1) * 32, col0 = (warp >> 1) * 16;
+    double* tile = a + static_cast<size_t>(I * kB + row0 + g) * ld + J * kB + col0 + 2 * m;
+    double2 v[4][2];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const double* row = a + static_cast<size_t>(I * kB + part(ty, i)) * ld + J * kB;
-        load4(row, tx, v[i]);
-    }
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            v[i][j] = *reinterpret_cast<const double2*>(tile + static_cast<size_t>(8 * i) * ld + 8 * j);
     __syncthreads();
-    double acc[4][4] = {};
-    tile_product(sw, kB, sp, kB, ty, tx, acc);
+    double acc[4][2][2] = {};
+#pragma unroll 4
+    for (int q = 0; q < kB; q += 4) {
+        const double* wr = sw + (q + m) * kUpdateLd + row0 + g;
+        const double* pr = sp + (q + m) * kUpdateLd + col0 + g;
+        double x[4], y[2];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        double* row = a + static_cast<size_t>(I * kB + part(ty, i)) * ld + J * kB;
+        for (int i = 0; i < 4; ++i) x[i] = wr[8 * i];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) v[i][j] -= acc[i][j];
-        *reinterpret_cast<double2*>(row + 2 * tx) = make_double2(v[i][0], v[i][1]);
-        *reinterpret_cast<double2*>(row + 32 + 2 * tx) = make_double2(v[i][2], v[i][3]);
-    }
-    if (I == J && I == k + 1) {
-        __syncthreads();   // smem becomes the pivot buffers
-        invert_block(v, ty, tx, smem, smem + 2 * kB, info);
+        for (int j = 0; j < 2; ++j) y[j] = pr[8 * j];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) d[part(ty, i) * kB + part(tx, j)] = v[i][j];
+            for (int j = 0; j < 2; ++j) mma_f64(acc[i][j], x[i], y[j]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            *reinterpret_cast<double2*>(tile + static_cast<size_t>(8 * i) * ld + 8 * j) =
+                make_double2(v[i][j].x - acc[i][j][0], v[i][j].y - acc[i][j][1]);
+    if (I == J && I == k + 1) {
+        __syncthreads();   // the tile is written; smem becomes the pivot buffers
+        const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+        double p[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) load4(a + static_cast<size_t>(I * kB + part(ty, i)) * ld + J * kB, tx, p[i]);
+        invert_block(p, ty, tx, smem, smem + 2 * kB, info);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) d[part(ty, i) * kB + part(tx, j)] = p[i][j];
     }
 }
 
@@ -320,7 +353,7 @@ SpdStatus spd_inverse(cfdxg_context* ctx, int n, const int* ro, const int* co, c
     k_spd_first_pivot<<<1, kThreads, 0, s>>>(a, np, d[0], w.info.get() + 1);
     check_launch(ctx);
     constexpr std::size_t kPanelSmem = sizeof(double) * (kB * kPanelLd + kB * kB);
-    constexpr std::size_t kUpdateSmem = sizeof(double) * 2 * kB * kB;
+    constexpr std::size_t kUpdateSmem = sizeof(double) * 2 * kB * kUpdateLd;
     CFDXG_CUDA(cudaFuncSetAttribute(k_spd_panel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(kPanelSmem)));
     CFDXG_CUDA(cudaFuncSetAttribute(k_spd_update, cudaFuncAttributeMaxDynamicSharedMemorySize,
