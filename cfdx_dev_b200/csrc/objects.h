@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "amg_setup.h"
+#include "cycle_tail.h"
 #include "dense.h"
 #include "device.cuh"
 
@@ -73,6 +74,10 @@ struct DevHierarchy {
     bool null_space = false;
     bool ns_in_order = false;
     DevBuf<double> ns_partials;
+    // FP64, default row order: the levels from tail_begin on run in one block
+    // (cycle_tail.cu); -1: none
+    int tail_begin = -1;
+    TailPlan tail;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     int64_t graph_kernels = 0;

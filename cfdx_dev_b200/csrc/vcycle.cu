@@ -40,7 +40,6 @@ constexpr int kT = 256;
 constexpr int kCoarseSweeps = 24;   // amg_preconditioner.h:2585
 constexpr int kFp32CoarsePre = 0;   // FP32 cycle on levels >= 1: V(0,1)
 constexpr int kFp32CoarsePost = 1;
-constexpr int kDenseDirectLimit = 16;
 
 template <class T>
 __device__ __forceinline__ bool finite_(T v) { return isfinite(v); }
@@ -313,73 +312,14 @@ __global__ void k_copy_cast(int n, const T* __restrict__ a, XO* __restrict__ b) 
     if (i < n) b[i] = static_cast<XO>(a[i]);
 }
 
-// Reference dense pivoted solve of the coarsest level (amg_preconditioner.h:2592-2663),
-// executed by one thread in the reference's order; under the constant null
-// space (ns = 1) the system is bordered by a row and a column of ones and the
-// mean of the solution is removed, summed in order.
+// Reference dense pivoted solve of the coarsest level (dense_lu_warp), one warp.
 template <class T>
 __global__ void k_dense_lu_reference(int n, const int* __restrict__ ro, const int* __restrict__ co,
                                      const T* __restrict__ va, const T* __restrict__ r,
                                      T* __restrict__ x, int ns, int* status) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    constexpr int kMax = kDenseDirectLimit + 1;
-    double m[kMax * kMax];
-    double b[kMax];
-    double sol[kMax];
-    const int sn = n + (ns ? 1 : 0);
-    for (int q = 0; q < sn * sn; ++q) m[q] = 0.0;
-    for (int i = 0; i < sn; ++i) b[i] = 0.0;
-    for (int i = 0; i < n; ++i) {
-        b[i] = static_cast<double>(r[i]);
-        for (int k = ro[i]; k < ro[i + 1]; ++k) m[i * sn + co[k]] += static_cast<double>(va[k]);
-    }
-    if (ns)
-        for (int i = 0; i < n; ++i) {
-            m[i * sn + n] = 1.0;
-            m[n * sn + i] = 1.0;
-        }
-    double matrix_scale = 0.0;
-    for (int q = 0; q < sn * sn; ++q) {
-        const double a = fabs(m[q]);
-        matrix_scale = (matrix_scale < a) ? a : matrix_scale;
-    }
-    const double pivot_tol = 128.0 * 2.220446049250313080847e-16 * (1.0 < matrix_scale ? matrix_scale : 1.0);
-    for (int k = 0; k < sn; ++k) {
-        int pivot = k;
-        double pivot_abs = fabs(m[k * sn + k]);
-        for (int i = k + 1; i < sn; ++i) {
-            const double c = fabs(m[i * sn + k]);
-            if (c > pivot_abs) { pivot_abs = c; pivot = i; }
-        }
-        if (!isfinite(pivot_abs) || pivot_abs <= pivot_tol) { atomicOr(status, kStatusNonFinite); return; }
-        if (pivot != k) {
-            for (int j = k; j < sn; ++j) { const double t = m[k * sn + j]; m[k * sn + j] = m[pivot * sn + j]; m[pivot * sn + j] = t; }
-            const double t = b[k]; b[k] = b[pivot]; b[pivot] = t;
-        }
-        const double diagonal = m[k * sn + k];
-        for (int i = k + 1; i < sn; ++i) {
-            const double factor = m[i * sn + k] / diagonal;
-            if (!isfinite(factor)) { atomicOr(status, kStatusNonFinite); return; }
-            m[i * sn + k] = 0.0;
-            for (int j = k + 1; j < sn; ++j) m[i * sn + j] -= factor * m[k * sn + j];
-            b[i] -= factor * b[k];
-        }
-    }
-    for (int ii = sn - 1; ii >= 0; --ii) {
-        double sum = b[ii];
-        for (int j = ii + 1; j < sn; ++j) sum -= m[ii * sn + j] * sol[j];
-        const double diagonal = m[ii * sn + ii];
-        if (!isfinite(diagonal) || fabs(diagonal) <= pivot_tol) { atomicOr(status, kStatusNonFinite); return; }
-        sol[ii] = sum / diagonal;
-        if (!isfinite(sol[ii])) { atomicOr(status, kStatusNonFinite); return; }
-    }
-    if (ns) {
-        double mean = 0.0;
-        for (int i = 0; i < n; ++i) mean += sol[i];
-        mean /= static_cast<double>(n);
-        for (int i = 0; i < n; ++i) sol[i] -= mean;
-    }
-    for (int i = 0; i < n; ++i) x[i] = static_cast<T>(sol[i]);
+    __shared__ LuScratch S;
+    const int lane = threadIdx.x;
+    if (!dense_lu_warp(S, n, ro, co, va, r, x, ns, lane) && lane == 0) atomicOr(status, kStatusNonFinite);
 }
 
 // x = Ainv * r: the inverse (formed in FP64) is read as FP32 -- half the bytes
@@ -865,12 +805,86 @@ void sweeps_from_zero(cfdxg_context* ctx, DevHierarchy<T>& d, DevLevel<T>& L, co
     L.xout = x;
 }
 
+// Compulsory bytes of one run of the tail: every level's operators once, the vectors in and out.
+inline double tail_cycle_bytes(const DevHierarchy<double>& d) {
+    double bytes = 16.0 * d.L[d.tail_begin].n;
+    for (int l = d.tail_begin; l < d.used; ++l) {
+        const DevLevel<double>& L = d.L[l];
+        bytes += nonzero_bytes(L) * L.nnz + row_bytes(L) * L.n + 8.0 * L.n +
+                 12.0 * static_cast<double>(L.p_col.size() + L.r_row.size());
+    }
+    return bytes;
+}
+
+// The levels that run in the tail: as many of the last ones as fit its threads
+// and registers and have at most kTailRows rows together (h: their rows'
+// lengths; a row or entry more per thread would have to be read again in every
+// sweep).  Not for the reference's row order nor under the constant null space
+// (its mean removals).
+void plan_tail(DevHierarchy<double>& d, const AmgHierarchy& h, bool reference_order) {
+    if (reference_order || d.null_space || d.coarse_mode == 2) return;
+    std::vector<int> longest(static_cast<std::size_t>(d.used), 0);
+    int begin = d.used;
+    int64_t rows = 0;
+    while (begin > 0 && d.used - begin < kTailMaxLevels && rows + d.L[begin - 1].n <= kTailRows) {
+        const DevLevel<double>& D = d.L[begin - 1];
+        const auto& ro = h.levels[begin - 1].A.ro;
+        int& most = longest[begin - 1];
+        for (int i = 0; i < D.n; ++i) most = std::max(most, static_cast<int>(ro[i + 1] - ro[i]));
+        if (!tail_fits(D.n, most, tail_threads_per_row(D.n, D.nnz))) break;
+        rows += D.n;
+        --begin;
+    }
+    if (begin == d.used) return;
+    d.tail_begin = begin;
+    TailPlan& P = d.tail;
+    P.levels = d.used - begin;
+    P.coarse_lu = d.coarse_mode == 1 ? 1 : 0;
+    P.coarse_sweeps = kCoarseSweeps;
+    P.omega = d.omega;
+    int at = 0;
+    for (int l = begin; l < d.used; ++l) {
+        const DevLevel<double>& D = d.L[l];
+        TailLevel& L = P.L[l - begin];
+        L.n = D.n;
+        L.ro = D.ro.get();
+        L.co = D.narrow ? nullptr : D.co.get();
+        L.co16 = D.narrow ? D.co16.get() : nullptr;
+        L.va = D.va.get();
+        L.inv_diag = D.inv_diag.get();
+        L.at = at;
+        at += 3 * D.n;
+        L.tpr = tail_threads_per_row(D.n, D.nnz);
+        L.parts = (longest[l] + L.tpr - 1) / L.tpr;
+        L.pre = l == 0 ? d.pre : d.coarse_pre;
+        L.post = l == 0 ? d.post : d.coarse_post;
+        if (l + 1 < d.used) {
+            L.p_off = D.p_off.get();
+            L.p_col = D.p_col.get();
+            L.p_val = D.p_val.get();
+            L.r_off = D.r_off.get();
+            L.r_row = D.r_row.get();
+            L.r_val = D.r_val.get();
+            const int64_t entries = static_cast<int64_t>(D.p_col.size());
+            L.tpr_r = tail_threads_per_row(d.L[l + 1].n, entries);
+            L.tpr_p = tail_threads_per_row(D.n, entries);
+        }
+    }
+}
+
 // Enqueue the cycle for levels [l, used) with the level-l right-hand side in L[l].r.
 template <class T>
 void enqueue_from(cfdxg_context* ctx, DevHierarchy<T>& d, int l) {
     cudaStream_t s = ctx->stream;
     DevLevel<T>& L = d.L[l];
-    const int gb = blocks_for(L.n, kT);
+    if constexpr (std::is_same<T, double>::value) {
+        if (l == d.tail_begin) {
+            account(tail_cycle_bytes(d));
+            launch_tail(ctx, d.tail, L.r.get(), L.x.get(), d.status);
+            L.xout = L.x.get();
+            return;
+        }
+    }
     if (l == d.used - 1) {
         if (d.coarse_mode == 1) {
             k_dense_lu_reference<T><<<1, 32, 0, s>>>(L.n, L.ro.get(), L.co.get(), L.va.get(), L.r.get(),
@@ -1328,6 +1342,7 @@ std::unique_ptr<DevHierarchy<T>> upload_hierarchy(cfdxg_context* ctx, const AmgH
             build_dense_inverse(ctx, *d, h.levels[used - 1]);
         }
     }
+    if constexpr (std::is_same<T, double>::value) plan_tail(*d, h, opt.reference_order);
     return d;
 }
 
@@ -1336,6 +1351,7 @@ std::unique_ptr<DevHierarchy<T>> upload_hierarchy(cfdxg_context* ctx, const AmgH
 template <class T>
 void set_hierarchy_values_device(cfdxg_context* ctx, DevHierarchy<T>& d, const DevRefresh& R, double omega) {
     d.omega = static_cast<T>(omega);
+    d.tail.omega = omega;
     for (int l = 0; l < d.used; ++l) {
         if (d.L[l].sparsified) {
             fill_sparsified(ctx, d.L[l], R.L[l], false);
@@ -1366,6 +1382,13 @@ void vcycle_apply(cfdxg_context* ctx, DevHierarchy<T>& d, const double* r, doubl
     cudaStream_t s = ctx->stream;
     DevLevel<T>& L = d.L[0];
     const int gb = blocks_for(L.n, kT);
+    if constexpr (std::is_same<T, double>::value) {
+        if (d.tail_begin == 0) {   // a small system: the whole cycle in one launch
+            ProfScope ps(ctx, "vcycle_tail_fp64", tail_cycle_bytes(d));
+            launch_tail(ctx, d.tail, r, z, d.status);
+            return;
+        }
+    }
     if (d.used == 1) {
         // single-level hierarchy: the coarsest treatment applies to the fine level
         launch_pdl(s, k_copy_cast<double, T>, gb, kT, L.n, r, L.r.get());
