@@ -701,6 +701,37 @@ def test_own_diagonal_cg_sizes(ctx, oracle, n):
         assert rel_l2(x, x_ref) <= 1e-12     # five updates of FP64 sums in another order
 
 
+def _graded_band(n):
+    """Symmetric, strictly diagonally dominant, rows of 1 to 10 entries."""
+    rows, cols = [], []
+    for k in range(1, 7):
+        i = np.arange(max(0, n - k))
+        i = i[i % 7 >= k]
+        rows += [i, i + k]
+        cols += [i + k, i]
+    rows, cols = np.concatenate(rows), np.concatenate(cols)
+    vals = -1.0 / np.abs(rows - cols)
+    diag = 1.0 + np.bincount(rows, -vals, minlength=n)
+    rows, cols = np.concatenate([rows, np.arange(n)]), np.concatenate([cols, np.arange(n)])
+    vals = np.concatenate([vals, diag])
+    order = np.lexsort((cols, rows))
+    ro = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=n))]).astype(np.int64)
+    return ro, cols[order].astype(np.int64), vals[order]
+
+
+@pytest.mark.parametrize("n", [9, 700, 75776, 75777])
+def test_own_diagonal_cg_row_lengths(ctx, oracle, n):
+    """Rows longer than the eight entries a thread holds, on either side of the
+    most rows it holds for (two blocks of 256 on each of 148 SMs)."""
+    ro, co, va = _graded_band(n)
+    b = np.random.default_rng(n).standard_normal(n)
+    x_ref, rep_ref = oracle.solve_cg(ro, co, va, b, "internal_jacobi", None, tolerance=1e-10)
+    x, rep = cg.solve_linear_system(cg.SparseMatrix.from_csr(ctx, ro, co, va), b, krylov="cg",
+                                    preconditioner="own_diagonal", tolerance=1e-10)
+    assert rep["status_name"] == "converged" and abs(rep["iterations"] - rep_ref["iterations"]) <= 2
+    assert rel_l2(x, x_ref) <= CG_LONG_TOL
+
+
 def test_own_diagonal_cg_refuses_negative_curvature(ctx):
     ro, co = np.array([0, 2, 4]), np.array([0, 1, 0, 1])
     A = cg.SparseMatrix.from_csr(ctx, ro, co, np.array([1.0, 2.0, 2.0, 1.0]))
