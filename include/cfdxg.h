@@ -283,7 +283,8 @@ typedef struct {
     int32_t precision;               /* CFDXG_PRECISION_* of the V-cycle */
     int32_t coarse_dense_limit;      /* FP32 V-cycle: the cycle ends at the first level with
                                         <= this many rows (6000) in a dense inverse, formed
-                                        in FP64 (LU with partial pivoting) and stored
+                                        in FP64 (symmetric sweeps; LU with partial
+                                        pivoting where those do not apply) and stored
                                         FP32; at 64^3 this is the 5,287-row level */
     int32_t reference_order;         /* 1: every row sum in CSR order, so the FP64
                                         V-cycle is bit-identical to the reference's;

@@ -739,6 +739,23 @@ def test_own_diagonal_cg_refuses_negative_curvature(ctx):
     assert rep["status_name"] == "not_applicable" and np.array_equal(x, np.zeros(2))
 
 
+@pytest.mark.parametrize("n", [1, 2, 1023, 4096, 4097, 8192, 8193])
+def test_gmres_orthogonalisation_sizes(ctx, oracle, n):
+    """Modified Gram-Schmidt in one block (four, then eight entries per thread)
+    and, above 8,192 rows, in a kernel per projection: the same iterates up to
+    the rounding of sums taken in another order."""
+    ro, co, va = _chain(n, 2.5)
+    b = np.random.default_rng(n).standard_normal(n)
+    x_ref, rep_ref = oracle.solve_gmres(ro, co, va, b, None, restart=20, tolerance=1e-8)
+    A = cg.SparseMatrix.from_csr(ctx, ro, co, va)
+    x, rep = cg.solve_gmres(A, b, restart=20, tolerance=1e-8)
+    assert rep["iterations"] == rep_ref["iterations"] and rel_l2(x, x_ref) <= REL_TOL
+    assert np.array_equal(x, cg.solve_gmres(A, b, restart=20, tolerance=1e-8)[0])
+    bad = b.copy()
+    bad[n // 2] = np.nan
+    assert cg.solve_gmres(A, bad, restart=20, tolerance=1e-8)[1]["status_name"] != "converged"
+
+
 @pytest.mark.parametrize("n_patches", [1, 32, 33, 40])
 def test_patch_tables_in_the_launch_and_on_the_device(ctx, oracle, n_patches):
     """Boundary faces spread over n_patches patches, every third fixed: up to
