@@ -543,6 +543,13 @@ int choose_tpr(int64_t nnz, int64_t rows, bool reference_order) {
     return tpr;
 }
 
+// Rows of sixteen entries or more on average, which share threads on any level
+// size: the ones whose values the FP32 cycle may hold as FP16 fractions.  Short
+// rows keep FP32 values, also where a small level gives them several threads.
+bool long_rows(int64_t nnz, int64_t rows, bool reference_order) {
+    return !reference_order && rows > 0 && static_cast<double>(nnz) / static_cast<double>(rows) >= 16.0;
+}
+
 // Threads per row of a sparsified smoothing operator (rows of 9-70 entries
 // at 64^3): the largest power of two up to a warp with at least
 // kSparseRowEntries entries per thread.  Eight measured 6.68 ms per 64^3 FP32
@@ -642,11 +649,12 @@ void upload_level(cfdxg_context* ctx, DevLevel<T>& D, const AmgLevel& H, bool wi
     // measured 10-20% slower (58.9 -> 70.6 us on the 77,039-row level), so
     // those keep int32 columns.
     upload_columns(ctx, D, H, with_transfer && opt.narrow_columns && D.tpr == 1);
-    // FP16 values on the shared-row levels (the dense coarse operators: 475 vs
+    // FP16 values on the long-row levels (the dense coarse operators: 475 vs
     // 501 us per FP32 cycle of levels >= 1 at 64^3, iterations unchanged); on
     // one-thread rows the conversion cost more than the bytes saved
     // (18.1 vs 17.7 us per fine-level sweep)
-    D.half = std::is_same<T, float>::value && opt.half_values && with_transfer && D.tpr > 1;
+    D.half = std::is_same<T, float>::value && opt.half_values && with_transfer &&
+             long_rows(D.nnz, D.n, opt.reference_order);
     upload_level_values(ctx, D, H);
     D.r.resize(D.n); D.x.resize(D.n); D.x2.resize(D.n); D.res.resize(D.n);
     if (with_transfer) {
@@ -1248,7 +1256,8 @@ void upload_level_device(cfdxg_context* ctx, DevLevel<T>& D, const AmgLevel& H, 
         device_copy(ctx, D.co, R.co.get(), D.nnz);
         D.co16.release();
     }
-    D.half = std::is_same<T, float>::value && opt.half_values && with_transfer && D.tpr > 1;
+    D.half = std::is_same<T, float>::value && opt.half_values && with_transfer &&
+             long_rows(D.nnz, D.n, opt.reference_order);
     if (D.half) {
         if constexpr (std::is_same<T, float>::value) {
             D.vh.resize(static_cast<std::size_t>(std::max(D.nnz, 1)));

@@ -756,6 +756,24 @@ def test_gmres_orthogonalisation_sizes(ctx, oracle, n):
     assert cg.solve_gmres(A, bad, restart=20, tolerance=1e-8)[1]["status_name"] != "converged"
 
 
+def test_short_rows_keep_fp32_values(ctx):
+    """Levels of under sixteen entries per row hold FP32 values in the FP32 cycle,
+    however many threads a row gets: with half_values off nothing changes."""
+    m = cases.simple_mesh(8)
+    mesh = cg.Mesh(ctx, m)
+    U, rAU, aP, p, fixed, value = cases.simple_fields(m, mesh.geometry()["cell_centres"])
+    A, b, _, _ = cg.assemble_pressure_correction(mesh, U, rAU, p, 1.0, fixed, value)
+    z = []
+    for half in (1, 0):
+        amg = cg.NativeBoomerAMGPreconditioner(ctx, precision="fp32_vcycle", max_levels=3, coarse_dense_limit=0,
+                                               coarse_drop_tolerance=0.0, half_values=half)
+        assert amg.setup(A)
+        sizes, nnz = amg.hierarchy_level_sizes(), amg.hierarchy_level_nnz()
+        assert len(sizes) == 3 and nnz[1] < 16 * sizes[1]
+        z.append(amg.apply(b))
+    assert np.array_equal(z[0], z[1])
+
+
 @pytest.mark.parametrize("n_patches", [1, 32, 33, 40])
 def test_patch_tables_in_the_launch_and_on_the_device(ctx, oracle, n_patches):
     """Boundary faces spread over n_patches patches, every third fixed: up to
