@@ -523,7 +523,10 @@ void launch_prolong(cfdxg_context* ctx, const DevLevel<T>& L, const T* xc, T* x,
 // thread's chain of loads: the rules below then give a row more threads (a
 // 53,937-row level of 31 entries per row: 17.8 us per FP64 sweep with two
 // threads per row; the 196,608-cell FP64 solve 12.05 -> 11.04 ms, the 215,622-cell
-// FP32 cycle 135 -> 126 us).
+// FP32 cycle 135 -> 126 us).  Down to one entry per thread on the Galerkin
+// levels: with four or more, the rows longer than the eight entries a lane has
+// loaded before the launch wait took two more latencies (2,058-cell FP64 solve
+// 1.99 -> 1.58 ms; 1.65 with two entries as the limit).
 constexpr double kFillThreads = 148.0 * 1024.0;
 
 // Threads per row of A: the largest power of two with at least eight entries
@@ -539,7 +542,7 @@ int choose_tpr(int64_t nnz, int64_t rows, bool reference_order) {
     while (tpr < 32 && avg >= 16.0 * tpr) tpr *= 2;
     while (tpr >= 32 && tpr < 128 && static_cast<double>(rows) * tpr < 2.0 * 148.0 * 2048.0 && avg >= 8.0 * tpr)
         tpr *= 2;
-    while (tpr < 32 && static_cast<double>(rows) * tpr < kFillThreads && avg >= 8.0 * tpr) tpr *= 2;
+    while (tpr < 32 && static_cast<double>(rows) * tpr < kFillThreads && avg >= 2.0 * tpr) tpr *= 2;
     return tpr;
 }
 
