@@ -316,19 +316,24 @@ __device__ __forceinline__ uint32_t ld32(const __nv_bfloat16* p) { return *reint
 
 // Inference rounds.  A warp owns 16 consecutive cells, rows g and g + 8 (g =
 // lane / 4) of the MMA tile, and the four lanes of a row (t = lane % 4) gather
-// its neighbours' states 16 bytes each: features 8 t .. 8 t + 7.  Contractions
-// do not depend on the order of their terms, so the features are numbered
-// within the MMA's k slots as the gather delivers them -- slot pairs (2 t, 2 t
-// + 1) and (2 t + 8, 2 t + 9) of k block q hold features 8 t + 4 q .. + 3 --
-// and the output columns so that a lane ends with features 8 t .. 8 t + 7 of
-// its two rows: [h, a] is the A operand straight from registers, the new state
-// leaves in 16-byte stores, and nothing passes through shared memory.  The
+// its neighbours' states 16 bytes each.  The state between rounds is stored in
+// the order in which the MMA's registers hold it: a lane's 16 bytes are
+// features 8 p + 2 t and 8 p + 2 t + 1, p = 0 .. 3 (lane_feature), its pairs of
+// k slots in the A operand and its columns of the result.  So [h, a] is the A
+// operand straight from registers, with feature f in k slot f; the new state
+// leaves in 16-byte stores, and nothing passes through shared memory.  (The k
+// slots matter: another assignment adds the FP32 products in another order,
+// which turned some BF16 roundings of the state over the rounds and moved the
+// result by 1.7e-4.)  The
 // weights stay in registers (48) over the warp's tiles, and a tile's couplings
 // are loaded one tile ahead.  Bound by the latency of the L2 gathers (some 400
 // bytes a cell and round): four rounds at 663,552 cells take 250 us; with 8
 // lanes of 8 bytes per row and the operands staged in shared memory 330.
 constexpr int kTileCells = 16;
 constexpr int kRoundThreads = 128;
+
+// feature q (0 .. 7) of lane t of a row
+__device__ __forceinline__ constexpr int lane_feature(int t, int q) { return 8 * (q >> 1) + 2 * t + (q & 1); }
 
 // x_i = [r_i / s, f_V, f_P, f_D] packed as one float4 per cell (k_encode's
 // input, 16 bytes), so the first round reads it instead of a 128-byte h0 row.
@@ -360,9 +365,10 @@ struct Encoder {
     __device__ __forceinline__ void load(const float* P, int t) {
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            b[q] = P[OFF_BIN + 8 * t + q];
+            const int f = lane_feature(t, q);
+            b[q] = P[OFF_BIN + f];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) w[q][c] = P[OFF_WIN + (8 * t + q) * 4 + c];
+            for (int c = 0; c < 4; ++c) w[q][c] = P[OFF_WIN + f * 4 + c];
         }
     }
     __device__ __forceinline__ void h0(float4 x, float (&f)[8]) const {
@@ -403,23 +409,21 @@ __global__ void __launch_bounds__(kRoundThreads, FIRST ? 2 : 4) k_round_gather_t
     const float* __restrict__ P, const double* __restrict__ rr, const double* __restrict__ diag,
     double* __restrict__ yout) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    // B operands: k slots numbered as above for W1 (k blocks 0, 1: h; 2, 3: a);
-    // W2 takes layer 1's output columns in their natural order and gives output
-    // column 8 j + n as feature 8 (n / 2) + 2 j + n % 2
+    // B operands (W1's k blocks 0, 1: h; 2, 3: a)
     uint32_t w1[4][4][2], w2[2][4][2];
 #pragma unroll
     for (int k = 0; k < 4; ++k)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const __nv_bfloat16* row = W1g + (8 * j + g) * (2 * F) + (k & 2) * (F / 2) + 8 * t + 4 * (k & 1);
+            const __nv_bfloat16* row = W1g + (8 * j + g) * (2 * F) + 16 * k + 2 * t;
             w1[k][j][0] = ld32(row);
-            w1[k][j][1] = ld32(row + 2);
+            w1[k][j][1] = ld32(row + 8);
         }
 #pragma unroll
     for (int k = 0; k < 2; ++k)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const __nv_bfloat16* row = W2g + (8 * (g >> 1) + 2 * j + (g & 1)) * F + 16 * k + 2 * t;
+            const __nv_bfloat16* row = W2g + (8 * j + g) * F + 16 * k + 2 * t;
             w2[k][j][0] = ld32(row);
             w2[k][j][1] = ld32(row + 8);
         }
@@ -543,7 +547,7 @@ __global__ void __launch_bounds__(kRoundThreads, FIRST ? 2 : 4) k_round_gather_t
         float out[4][4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const float2 b2 = *reinterpret_cast<const float2*>(Pr + OFF_B2 + 8 * t + 2 * j);
+            const float2 b2 = *reinterpret_cast<const float2*>(Pr + OFF_B2 + 8 * j + 2 * t);
             out[j][0] = b2.x + hv[0][2 * j];
             out[j][1] = b2.y + hv[0][2 * j + 1];
             out[j][2] = b2.x + hv[1][2 * j];
@@ -563,7 +567,7 @@ __global__ void __launch_bounds__(kRoundThreads, FIRST ? 2 : 4) k_round_gather_t
             float ya = 0.0f, yb = 0.0f;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const float wo0 = P[OFF_WOUT + 8 * t + 2 * j], wo1 = P[OFF_WOUT + 8 * t + 2 * j + 1];
+                const float wo0 = P[OFF_WOUT + 8 * j + 2 * t], wo1 = P[OFF_WOUT + 8 * j + 2 * t + 1];
                 ya += wo0 * out[j][0] + wo1 * out[j][1];
                 yb += wo0 * out[j][2] + wo1 * out[j][3];
             }

@@ -124,6 +124,24 @@ def test_inference_tiles_and_neighbour_counts(ctx, kind):
     assert np.linalg.norm(y - y_ref) <= 3e-2 * np.linalg.norm(y_ref)
 
 
+@pytest.mark.parametrize("kind", ["tet3", "layer4"])
+def test_inference_adds_the_features_in_their_order(ctx, kind):
+    """Outputs recorded with kernels that staged [h, a] in shared memory by
+    feature number: the MMA's FP32 sums depend on which k slot a feature takes.
+    Any other FP32 sum shows in a cell's value as at least 2^-24 of it; what
+    remains (the norm of r, the diagonal) is FP64."""
+    m = cases.simple_mesh(3) if kind == "tet3" else cg.boundary_layer_case(4, 3, 5)
+    mesh = cg.Mesh(ctx, m)
+    U, rAU, aP, p, fixed, value = cases.simple_fields(m, mesh.geometry()["cell_centres"])
+    A, b, phi, grad = cg.assemble_pressure_correction(mesh, U, rAU, p, 1.0, fixed, value)
+    net = cg.LearnedPreconditioner(ctx, seed=3)
+    net.bind(mesh, A, aP)
+    net.set_parameters(mo.init_params(5).astype(np.float32))
+    y = net.apply(np.random.default_rng(4).standard_normal(A.n))
+    with np.load(cases.ROOT / "tests" / "golden" / "mpnn_inference.npz") as recorded:
+        assert np.allclose(y, recorded[kind], rtol=1e-9, atol=0)
+
+
 def test_training_reduces_loss_and_weights_roundtrip(bound, tmp_path):
     G, net = bound["G"], bound["net"]
     R, E = _pairs(G, 4, seed=1)
