@@ -1015,7 +1015,7 @@ __global__ void k_cg_direction(int n, double* __restrict__ p, const double* __re
 // residual outside the range in which plain squares are exact enough) it stops
 // before x changes again and the host decides on that iteration.
 enum CgRunSlot : int {
-    kRunCode = 20, kRunIterations = 21, kRunPAp = 22, kRunRsOld = 23, kRunRsNew = 24, kRunRR = 25, kRunXBad = 26,
+    kRunCode = 20, kRunDone = 21, kRunPAp = 22, kRunRsOld = 23, kRunRsNew = 24, kRunRR = 25, kRunXBad = 26,
     kRunZBad = 27, kRunP = 28, kRunCount = 29
 };
 enum CgRunCode : int { kRunDecide = 0, kRunCurvature = 1, kRunStalled = 2 };
@@ -1023,6 +1023,14 @@ constexpr int kRunThreads = kT;
 constexpr int kRunBlocksPerSm = 3;   // 80 registers; four per SM spilled
 constexpr int kHeldBlocksPerSm = 2;  // with the thread's row in registers
 constexpr int kHeldEntries = 8;
+// Iterations of one launch; the host relaunches a solve that needs more.  The
+// barriers' counter grows by the grid's blocks twice an iteration and must not
+// wrap within a launch (the largest grids did after some 4.8 million
+// iterations, and a barrier whose target had wrapped let its blocks pass).
+// A relaunch costs some 50 us in half a second.
+constexpr int kRunIterations = 1 << 16;
+constexpr int kRunMostBlocks = 8192;
+static_assert((2ull * kRunIterations + 1) * kRunMostBlocks < (1ull << 31), "the arrival counter wraps");
 // A barrier gives up after this many polls (about a second): the blocks are
 // co-resident, so only a failure elsewhere on the GPU could keep one away.
 constexpr unsigned kRunSpinLimit = 1u << 20;
@@ -1252,7 +1260,7 @@ __global__ void __launch_bounds__(kRunThreads, HELD ? kHeldBlocksPerSm : kRunBlo
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         slots[kRunCode] = code;
-        slots[kRunIterations] = it - 1;
+        slots[kRunDone] = it - 1;
         slots[kRunPAp] = pAp;
         slots[kRunRsOld] = rsold;
         slots[kRunRsNew] = rsnew;
@@ -1899,14 +1907,14 @@ KrylovResult cg_solve(cfdxg_context* ctx, const cfdxg_matrix* A, const double* b
         // a row per thread, held in registers, while the GPU has that many threads; above that the loop
         const bool hold = blocks_for(n, kRunThreads) <=
                           std::min(kHeldBlocksPerSm, resident_per_sm<k_cg_run<true>>()) * ctx->sm_count;
-        const int blocks = std::min(blocks_for(n, kRunThreads),
-                                    hold ? blocks_for(n, kRunThreads)
-                                         : std::min(kRunBlocksPerSm, resident_per_sm<k_cg_run<false>>()) * ctx->sm_count);
+        const int looped = std::min(kRunBlocksPerSm, resident_per_sm<k_cg_run<false>>()) * ctx->sm_count;
+        const int blocks = std::min(kRunMostBlocks, hold ? blocks_for(n, kRunThreads)
+                                                         : std::min(blocks_for(n, kRunThreads), looped));
         const void* kernel = hold ? reinterpret_cast<const void*>(k_cg_run<true>)
                                   : reinterpret_cast<const void*>(k_cg_run<false>);
         while (done < max_iter) {
             CFDXG_CUDA(cudaMemsetAsync(ctx->scratch.ticket + 4, 0, sizeof(unsigned), ctx->stream));
-            const int limit = static_cast<int>(std::min<int64_t>(max_iter - done, 1 << 30));
+            const int limit = static_cast<int>(std::min<int64_t>(max_iter - done, kRunIterations));
             {
                 ProfScope ps(ctx, "cg_own_diagonal", 0.0);
                 int nn = ni;
@@ -1925,7 +1933,7 @@ KrylovResult cg_solve(cfdxg_context* ctx, const cfdxg_matrix* A, const double* b
             E.fetch(kRunCount);
             const double res = E.host(kCgRes);
             const int code = static_cast<int>(E.host(kRunCode));
-            const int64_t ran = static_cast<int64_t>(E.host(kRunIterations));
+            const int64_t ran = static_cast<int64_t>(E.host(kRunDone));
             if (code == kRunStalled) throw Error(CFDXG_ERR_CUDA, "CG: a grid-wide barrier was not reached in time");
             done += ran;
             result.preconditioner_applications += ran;

@@ -732,6 +732,22 @@ def test_own_diagonal_cg_row_lengths(ctx, oracle, n):
     assert rel_l2(x, x_ref) <= CG_LONG_TOL
 
 
+def test_own_diagonal_cg_over_several_launches(ctx):
+    """More iterations than one launch takes (65,536), on a chain whose first
+    row alone has a source: k iterations solve its first k rows, so x_i =
+    (k - i) / (k + 1) and each iteration leaves a residual of 1 / (k + 1)."""
+    n, k = 70000, 65600
+    ro, co, va = _chain(n, 2.0)
+    b = np.zeros(n)
+    b[0] = 1.0
+    x, rep = cg.solve_linear_system(cg.SparseMatrix.from_csr(ctx, ro, co, va), b, krylov="cg",
+                                    preconditioner="own_diagonal", tolerance=1e-10, max_iterations=k)
+    assert rep["iterations"] == k and rep["status_name"] == "max_iter_reached"
+    exact = np.maximum(k - np.arange(n), 0) / (k + 1.0)
+    # a rounding of each of the k updates of an entry
+    assert np.abs(x - exact).max() <= 2 * k * 2.0 ** -53
+
+
 def test_own_diagonal_cg_refuses_negative_curvature(ctx):
     ro, co = np.array([0, 2, 4]), np.array([0, 1, 0, 1])
     A = cg.SparseMatrix.from_csr(ctx, ro, co, np.array([1.0, 2.0, 2.0, 1.0]))
