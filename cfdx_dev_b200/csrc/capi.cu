@@ -257,6 +257,13 @@ extern "C" int cfdxg_context_destroy(cfdxg_context* ctx) {
     return CFDXG_OK;
 }
 
+// Not part of the ABI: the tests make a kernel's wait run out with no polls.
+extern "C" int cfdxg_internal_wait_polls(cfdxg_context* ctx, uint32_t polls) {
+    if (!ctx) return CFDXG_ERR_INVALID_ARGUMENT;
+    ctx->wait_polls = polls;
+    return CFDXG_OK;
+}
+
 extern "C" const char* cfdxg_last_error(const cfdxg_context* ctx) { return ctx ? ctx->error.c_str() : "null context"; }
 extern "C" int64_t cfdxg_kernel_launches(const cfdxg_context* ctx) { return ctx ? ctx->launches : 0; }
 extern "C" void* cfdxg_context_stream(const cfdxg_context* ctx) {

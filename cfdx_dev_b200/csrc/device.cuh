@@ -113,6 +113,7 @@ struct cfdxg_context {
     int64_t launches = 0;
     cfdxg::Scratch scratch;
     int sm_count = 148;
+    unsigned wait_polls = 1u << 20;   // polls after which a kernel's wait gives up (near a second)
     std::shared_ptr<void> krylov_workspace;   // grown on demand by the Krylov driver
     cfdxg::Profiler prof;
     cfdxg::StagingPool staging;

@@ -1035,15 +1035,15 @@ constexpr int kHeldEntries = 8;
 constexpr int kRunIterations = 1 << 16;
 constexpr int kRunMostBlocks = 8192;
 static_assert((2ull * kRunIterations + 1) * kRunMostBlocks < (1ull << 31), "the arrival counter wraps");
-// A barrier gives up after this many polls (about a second): the blocks are
-// co-resident, so only a failure elsewhere on the GPU could keep one away.
-constexpr unsigned kRunSpinLimit = 1u << 20;
 
 // Sums v[0..NS) and takes the maximum of v[NS..NV) over the grid; every thread
 // gets the results.  Also a grid-wide barrier: what the block's threads wrote
-// before it is visible to every block after it.  Returns false when it gave up.
+// before it is visible to every block after it.  Returns false when a warp has
+// polled poll_limit times: the blocks are co-resident, so only a failure
+// elsewhere on the GPU could keep one away (cfdxg_context::wait_polls).
 template <int NS, int NV>
-__device__ __forceinline__ bool grid_combine(double (&v)[NV], double* part, unsigned* counter, unsigned target) {
+__device__ __forceinline__ bool grid_combine(double (&v)[NV], double* part, unsigned* counter, unsigned target,
+                                             unsigned poll_limit) {
     constexpr int kW = kRunThreads / 32;
     __shared__ double sm[NV][kW];
     __shared__ double total[NV];
@@ -1075,10 +1075,9 @@ __device__ __forceinline__ bool grid_combine(double (&v)[NV], double* part, unsi
     // a warp per result waits for all blocks by itself, so that it can go on to their partials at once;
     // its acquire and the barrier below order the other blocks' writes before what the block reads next
     if (warp < NV) {
-        unsigned seen = 0, polls = 0;
-        do {
+        unsigned seen = 0;
+        for (unsigned polls = 0; seen < target && polls < poll_limit; ++polls)
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
-        } while (seen < target && ++polls < kRunSpinLimit);
         if (__any_sync(0xffffffffu, seen < target)) gave_up = 1;
         double t = 0.0;
         for (int b = lane; b < static_cast<int>(gridDim.x); b += 32) {
@@ -1114,7 +1113,8 @@ template <bool HELD>
 __global__ void __launch_bounds__(kRunThreads, HELD ? kHeldBlocksPerSm : kRunBlocksPerSm) k_cg_run(
     int n, const int* __restrict__ ro, const int* __restrict__ co, const double* __restrict__ va,
     const double* __restrict__ b, const double* __restrict__ d, double* x, double* r, double* z, double* p0, double* p1,
-    double* Ap, double rsold, double tol_abs, int limit, double* part, unsigned* counter, double* slots) {
+    double* Ap, double rsold, double tol_abs, int limit, unsigned poll_limit, double* part, unsigned* counter,
+    double* slots) {
     const int stride = gridDim.x * kRunThreads;
     const int first_row = blockIdx.x * kRunThreads + threadIdx.x;
     double* half[2] = {part, part + 4 * gridDim.x};
@@ -1207,7 +1207,7 @@ __global__ void __launch_bounds__(kRunThreads, HELD ? kHeldBlocksPerSm : kRunBlo
             pn = t;
         }
         arrivals += gridDim.x;
-        if (!grid_combine<2, 3>(s1, half[0], counter, arrivals)) {
+        if (!grid_combine<2, 3>(s1, half[0], counter, arrivals, poll_limit)) {
             code = kRunStalled;
             break;
         }
@@ -1252,7 +1252,7 @@ __global__ void __launch_bounds__(kRunThreads, HELD ? kHeldBlocksPerSm : kRunBlo
             if (!isfinite(zi)) s2[3] = 1.0;
         }
         arrivals += gridDim.x;
-        if (!grid_combine<2, 4>(s2, half[1], counter, arrivals)) {
+        if (!grid_combine<2, 4>(s2, half[1], counter, arrivals, poll_limit)) {
             code = kRunStalled;
             break;
         }
@@ -1928,7 +1928,8 @@ KrylovResult cg_solve(cfdxg_context* ctx, const cfdxg_matrix* A, const double* b
                        *part = ws.mpartial.get(), *slots = E.slot(0);
                 unsigned* counter = ctx->scratch.ticket + 4;
                 void* args[] = {&nn, &ro, &co, &va, &b, &own_diagonal, &x, &r, &zz, &p0, &p1, &ap, &rsold,
-                                const_cast<double*>(&tol_abs), const_cast<int*>(&limit), &part, &counter, &slots};
+                                const_cast<double*>(&tol_abs), const_cast<int*>(&limit), &ctx->wait_polls, &part,
+                                &counter, &slots};
                 CFDXG_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(kRunThreads), args, 0, ctx->stream));
                 check_launch(ctx);
             }
@@ -1938,7 +1939,8 @@ KrylovResult cg_solve(cfdxg_context* ctx, const cfdxg_matrix* A, const double* b
             const double res = E.host(kCgRes);
             const int code = static_cast<int>(E.host(kRunCode));
             const int64_t ran = static_cast<int64_t>(E.host(kRunDone));
-            if (code == kRunStalled) throw Error(CFDXG_ERR_CUDA, "CG: a grid-wide barrier was not reached in time");
+            if (code == kRunStalled)   // x: some entries one update further than others
+                throw Error(CFDXG_ERR_CUDA, "CG: a grid-wide barrier was not reached in time; x holds no iterate");
             done += ran;
             result.preconditioner_applications += ran;
             if (code == kRunCurvature) {

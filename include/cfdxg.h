@@ -459,7 +459,10 @@ int cfdxg_request_default(cfdxg_request* req);
  * or a diagonal that is not positive, returns CFDXG_NOT_APPLICABLE with x
  * untouched (linear_solver_dispatch.h:259-267); its AMG keeps the smoother
  * certificate and is set up only when the initial residual has not already
- * converged.  CG takes no learned stage. */
+ * converged.  CG takes no learned stage.  CG with OWN_DIAGONAL iterates in one
+ * launch whose blocks wait for one another, each wait limited to near a second:
+ * one that runs out returns CFDXG_ERR_CUDA, and x in device memory then holds
+ * no iterate. */
 int cfdxg_solve_linear_system(cfdxg_context* ctx, const cfdxg_matrix* A, const double* rhs,
                               double* x, int32_t mem, const cfdxg_request* req,
                               int64_t max_iterations, double tolerance, cfdxg_report* report);

@@ -748,6 +748,24 @@ def test_own_diagonal_cg_over_several_launches(ctx):
     assert np.abs(x - exact).max() <= 2 * k * 2.0 ** -53
 
 
+@pytest.mark.parametrize("n", [300, 70000, 80000])
+def test_own_diagonal_cg_gives_up_waiting(n):
+    """A barrier whose wait runs out (no polls at all) ends the solve with an
+    error, for rows held in registers and for the loop; the context goes on."""
+    ctx = cg.Context(0)
+    ro, co, va = _chain(n)
+    A = cg.SparseMatrix.from_csr(ctx, ro, co, va)
+    b = np.random.default_rng(n).standard_normal(n)
+    kw = dict(krylov="cg", preconditioner="own_diagonal", tolerance=1e-10)
+    assert ctx.lib.cfdxg_internal_wait_polls(ctx.handle, 0) == 0
+    with pytest.raises(cg.CfdxgError, match="barrier was not reached"):
+        cg.solve_linear_system(A, b, **kw)
+    assert ctx.lib.cfdxg_internal_wait_polls(ctx.handle, 1 << 20) == 0
+    x, rep = cg.solve_linear_system(A, b, **kw)
+    assert rep["status_name"] == "converged"
+    assert np.linalg.norm(A.matvec(x) - b) <= 2e-10 * np.linalg.norm(b)
+
+
 def test_own_diagonal_cg_refuses_negative_curvature(ctx):
     ro, co = np.array([0, 2, 4]), np.array([0, 1, 0, 1])
     A = cg.SparseMatrix.from_csr(ctx, ro, co, np.array([1.0, 2.0, 2.0, 1.0]))
