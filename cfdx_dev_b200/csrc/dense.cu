@@ -350,6 +350,11 @@ SpdStatus spd_inverse(cfdxg_context* ctx, int n, const int* ro, const int* co, c
     const int t32 = (n + 31) / 32;
     k_symmetry_check<<<dim3(t32, t32), 256, 0, s>>>(n, np, a, w.info.get());
     check_launch(ctx);
+    // one wait here, for the caller's other route not to pay the sweeps as well
+    int info[2] = {0, 0};
+    CFDXG_CUDA(cudaMemcpyAsync(info, w.info.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
+    CFDXG_CUDA(cudaStreamSynchronize(s));
+    if (info[0]) return SpdStatus::kNotSymmetric;
     k_spd_first_pivot<<<1, kThreads, 0, s>>>(a, np, d[0], w.info.get() + 1);
     check_launch(ctx);
     constexpr std::size_t kPanelSmem = sizeof(double) * (kB * kPanelLd + kB * kB);
@@ -380,10 +385,8 @@ SpdStatus spd_inverse(cfdxg_context* ctx, int n, const int* ro, const int* co, c
     if (out64) k_negated_symmetric<double><<<dim3(t32, t32), 256, 0, s>>>(n, np, ld_out, a, out64);
     else k_negated_symmetric<float><<<dim3(t32, t32), 256, 0, s>>>(n, np, ld_out, a, out32);
     check_launch(ctx);
-    int info[2] = {0, 0};
     CFDXG_CUDA(cudaMemcpyAsync(info, w.info.get(), 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
     CFDXG_CUDA(cudaStreamSynchronize(s));
-    if (info[0]) return SpdStatus::kNotSymmetric;
     return info[1] ? SpdStatus::kNotPositive : SpdStatus::kInverted;
 }
 

@@ -7,7 +7,8 @@ namespace cfdxg {
 constexpr int kSpdBlock = 64;
 
 // Work arrays, kept with the hierarchy for its refreshes: the matrix padded to
-// whole blocks, two panels and two pivot blocks, and the status words.
+// whole blocks (the LU route's too), two panels and two pivot blocks, and the
+// status words.
 struct SpdWorkspace {
     DevBuf<double> a, panels;
     DevBuf<int> info;
@@ -17,9 +18,9 @@ enum class SpdStatus { kInverted, kNotSymmetric, kNotPositive };
 
 // The inverse of the n x n matrix given by its device CSR (unique columns),
 // row-major (leading dimension ld_out) into out64, or rounded into out32 when
-// out64 is null.  A matrix
-// that is not symmetric to rounding, or not positive definite, is reported
-// and leaves the output undefined.  Synchronises the stream.
+// out64 is null.  A matrix that is not symmetric to rounding is reported before
+// any sweep, one that is not positive definite after them; either leaves the
+// output undefined.  Synchronises the stream.
 SpdStatus spd_inverse(cfdxg_context* ctx, int n, const int* ro, const int* co, const double* va, SpdWorkspace& w,
                       int ld_out, float* out32, double* out64);
 

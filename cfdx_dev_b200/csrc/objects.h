@@ -67,7 +67,7 @@ struct DevHierarchy {
     // the dense inverse's work arrays and LU solver handle, kept for refreshes
     SpdWorkspace spd;
     std::shared_ptr<void> solver;
-    DevBuf<double> lu_a, lu_x, lu_work;
+    DevBuf<double> lu_x, lu_work;   // the LU route factors in spd.a
     DevBuf<int> lu_ipiv, lu_info;
     // constant null space: the cycle's mean removals (in index order with
     // reference_order) and the bordered coarsest solve

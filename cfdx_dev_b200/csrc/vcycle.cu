@@ -726,10 +726,11 @@ void build_dense_inverse_dev(cfdxg_context* ctx, DevHierarchy<T>& d, int n, cons
         std::fprintf(stderr, "[cfdxg setup] dense coarse inverse of %d rows by LU (%s)\n", N,
                      d.null_space ? "bordered"
                                   : (spd == SpdStatus::kNotSymmetric ? "not symmetric" : "not positive definite"));
-    // the work arrays and the solver handle stay with the hierarchy for its refreshes
-    DevBuf<double>& at = d.lu_a;
+    // the work arrays and the solver handle stay with the hierarchy for its
+    // refreshes; the matrix goes where the symmetric route would have it
+    DevBuf<double>& at = d.spd.a;
     DevBuf<double>& x = d.lu_x;
-    at.resize(NN);
+    if (at.size() < NN) at.resize(NN);
     d.lu_ipiv.resize(N);
     d.lu_info.resize(1);
     const int64_t grid_nn = blocks_for(static_cast<int64_t>(NN), kT);

@@ -46,6 +46,39 @@ def test_dense_inverse_of_an_spd_level(ctx, n, dense_fp64):
     assert np.linalg.norm(amg.apply(r) - 0.5 * z) <= 40 * 2.0 ** -23 * np.linalg.norm(0.5 * z)
 
 
+def test_nonsymmetric_level_pays_for_lu_alone(ctx):
+    """A refresh of a level that is not symmetric launches none of the two
+    kernels per 64 columns of the symmetric route, and keeps two n x n FP64
+    arrays beside the FP32 inverse and the solver's own memory (315 MB here);
+    a third would be 128 MB more."""
+    import torch
+    n = 4000
+    i = np.arange(n)
+    a = np.zeros((n, n))
+    a[i, i] = 3.0
+    a[i[1:], i[:-1]] = a[i[:-1], i[1:]] = -1.0
+    launches = {}
+    for skew in (0.0, 0.3):
+        a[0, 1] = -1.0 - skew
+        rows, cols = np.nonzero(a)
+        ro = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=n))]).astype(np.int64)
+        A = cg.SparseMatrix.from_csr(ctx, ro, cols.astype(np.int64), a[rows, cols])
+        r = np.random.default_rng(7).standard_normal(n)
+        z = np.linalg.solve(a, r)
+        for _ in range(2):   # the first one loads the solver's own code
+            free = torch.cuda.mem_get_info()[0]
+            amg = cg.NativeBoomerAMGPreconditioner(ctx, precision="fp32_vcycle")
+            assert amg.setup(A), amg.last_error()
+            used = free - torch.cuda.mem_get_info()[0]
+            before = ctx.kernel_launches
+            assert amg.update_values(A)
+            launches[skew] = ctx.kernel_launches - before
+            assert np.linalg.norm(amg.apply(r) - z) <= 40 * 2.0 ** -23 * np.linalg.norm(z)
+            del amg
+    assert launches[0.3] < launches[0.0] - 100
+    assert used <= (2 * 8 + 4) * n * n + 380e6
+
+
 def test_dense_inverse_of_a_nonsymmetric_level(ctx):
     """Not symmetric: the LU route, with the same result."""
     a, ro, co, va = _system(200, 3, 1.0, skew=0.3)
