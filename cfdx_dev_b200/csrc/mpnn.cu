@@ -1388,10 +1388,15 @@ extern "C" int cfdxg_mpnn_bind(cfdxg_context* ctx, cfdxg_mpnn* net, cfdxg_mesh* 
         for (int64_t i = 0; i < n; ++i) mean += logs[i];
         mean /= n;
         for (int64_t i = 0; i < n; ++i) sq += (logs[i] - mean) * (logs[i] - mean);
-        const double sd = std::sqrt(sq / n);
+        // On a uniform mesh the logarithms differ by rounding alone (some 1e-15,
+        // more on finer lattices), which a division by its own deviation would
+        // turn into inputs of size one: a constant is left at its distance from
+        // the mean, next to zero.
+        const double deviation = std::sqrt(sq / n);
+        const double sd = deviation > 1e-12 * std::max(1.0, std::abs(mean)) ? deviation : 1.0;
         rows([&](int64_t b, int64_t e) {
             for (int64_t i = b; i < e; ++i)
-                feats[slot * n + i] = static_cast<float>((logs[i] - mean) / (sd > 0.0 ? sd : 1.0));
+                feats[slot * n + i] = static_cast<float>((logs[i] - mean) / sd);
         });
     };
     rows([&](int64_t b, int64_t e) {

@@ -74,8 +74,9 @@ class Graph:
 
         def standard(v):
             lv = np.log(v)
-            sd = lv.std()
-            return (lv - lv.mean()) / (sd if sd > 0 else 1.0)
+            mean, sd = lv.mean(), lv.std()
+            # rounding alone (a uniform mesh) is no variation
+            return (lv - mean) / (sd if sd > 1e-12 * max(1.0, abs(mean)) else 1.0)
         self.feats = np.stack([standard(volume), standard(a_p), standard(diag)], axis=1)
 
     def matvec(self, x):

@@ -101,14 +101,16 @@ def test_tensor_core_inference_matches_oracle(bound):
     assert np.allclose(net.apply(2.0 * r), 2.0 * y, rtol=1e-5, atol=1e-12 * np.abs(y).max())
 
 
-@pytest.mark.parametrize("kind", ["layer2", "tet3", "tet7", "layer4", "layer9"])
+@pytest.mark.parametrize("kind", ["layer2", "tet1", "tet3", "tet7", "layer4", "layer9", "hex4", "hex16"])
 def test_inference_tiles_and_neighbour_counts(ctx, kind):
     """Fewer cells than a 16-cell tile, remainder tiles, more than four
     neighbours per cell; the same bound as above (BF16 operands and state).
-    Not a uniform lattice: its log volumes differ by rounding alone (their
-    standard deviation is 6e-16), which the standardised input divides by."""
+    On the uniform lattices the log volumes differ by rounding alone (their
+    standard deviation is 6e-16): that input is constant."""
     if kind.startswith("tet"):
         m = cases.simple_mesh(int(kind[3:]))
+    elif kind.startswith("hex"):
+        m = cg.hex_case(*{"hex4": (4, 3, 5), "hex16": (16, 16, 16)}[kind])
     else:
         m = cg.boundary_layer_case(*{"layer2": (2, 3, 2), "layer4": (4, 3, 5), "layer9": (9, 13, 7)}[kind])
     mesh = cg.Mesh(ctx, m)
