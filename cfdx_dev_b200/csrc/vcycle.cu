@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(kT) k_dense_inverse_apply(int n, int ld, const
     pdl_trigger();
     const int row0 = blockIdx.x * kDenseRows;
     int c = threadIdx.x * V;
-    S m[kDenseRows][V];
+    alignas(16) S m[kDenseRows][V];
     const auto load = [&](int at) {
 #pragma unroll
         for (int q = 0; q < kDenseRows; ++q) {
