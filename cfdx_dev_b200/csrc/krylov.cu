@@ -396,7 +396,7 @@ __device__ __forceinline__ void grid_multi_sum(const double (&acc)[C], double ex
     }
 }
 
-// The fused passes are instantiated for each basis count C (1..kChunk): the
+// The fused passes are instantiated for each basis count C (1..kFused): the
 // per-vector accumulators and loads take exactly C registers' worth, so the
 // small counts of the first Arnoldi steps run at higher occupancy.
 

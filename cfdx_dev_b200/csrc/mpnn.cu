@@ -85,12 +85,6 @@ namespace {
 
 using namespace mp;
 
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 // x = [r/s, feats]; h0 = relu(W_in x + b_in) of the pairs' cells (pair s holds
 // cells [s n, (s+1) n)).  Eight lanes per cell, each lane four features (one
 // 16-byte store); the group's first lane forms r/s.
