@@ -17,8 +17,10 @@
 // Two launches per 64-wide block column: the panel (P = A_:k, W = P D, both
 // left transposed for the next kernel) and the rank-64 update of the lower
 // tiles, whose first block also inverts the next pivot block, so that the
-// serial part hides behind the update.  Bound by FP64 multiply-adds (n^3 of
-// them in all) on large levels and by the serial pivots on small ones.  3,429
+// serial part hides behind the update: n^3 / 2 multiply-adds in the updates, 64
+// n^2 in the panels.  An update takes 20 us at 500 rows, where the serial pivots
+// (19 alone) are all of it, 27 at 2,000, 43 at 3,429 (FP64 tensor cores 52%
+// busy) and 95 at 5,287, where the products bound it; a panel 11 to 17.  3,429
 // rows: 3.2 ms, against 10.5 ms by cuSOLVER's potrf and potri, whose triangular
 // inverse and product run in many small kernels.
 #include "dense.h"
@@ -183,7 +185,7 @@ __device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
 // four k: six shared reads (two wavefronts each, kUpdateLd spreading the four k
 // over the banks) for 2,048 multiply-adds.  With 4 x 4 register tiles a thread's
 // shared reads took as long as its multiply-adds: 63 us a launch at 3,429 rows
-// against 43, of which block 0's serial pivots are most.
+// against 43.
 constexpr int kUpdateLd = kB + 4;
 __global__ void __launch_bounds__(kThreads, 3) k_spd_update(double* a, int ld, int tiles, int k,
                                                             const double* pt, const double* wt, double* d, int* info) {

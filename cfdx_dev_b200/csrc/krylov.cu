@@ -170,7 +170,8 @@ __global__ void k_axpy_absmax(int n, double* __restrict__ w, const double* __res
 // On systems of a few thousand rows each of the 2 (j + 1) projections of step j
 // is less than a microsecond of work and took 3.9 us as a kernel.  Here one
 // block keeps w in registers over all of them, with the next basis vector's
-// loads in flight during the reduction.  Bound by the block-wide sums.  FP64
+// loads in flight during the reduction.  Bound by the one SM's issue slots (65%
+// busy) and the block-wide sums.  FP64
 // GMRES of 2,058 cells: 2.23 -> 1.99 ms, of 7,986: 3.04 -> 2.76 (8,192 rows fill
 // the registers).
 constexpr int kSmallThreads = 1024;
@@ -1109,6 +1110,9 @@ __device__ __forceinline__ bool grid_combine(double (&v)[NV], double* part, unsi
 // same operations in the same order.  Bound by the two grid-wide sums; 32,768
 // rows of the Poisson driver, 263 iterations: 3.70 ms with the loop and fences
 // around the counter, 3.35 held, 3.1 with one release and acquire in their place.
+// The loop, on more rows, is bound by its three gathers an entry from L2: 1,331,000
+// hexahedra 85 us an iteration, 4,194,304 of a boundary layer 237, where separate
+// kernels with a read-back took 146 and 308.
 template <bool HELD>
 __global__ void __launch_bounds__(kRunThreads, HELD ? kHeldBlocksPerSm : kRunBlocksPerSm) k_cg_run(
     int n, const int* __restrict__ ro, const int* __restrict__ co, const double* __restrict__ va,

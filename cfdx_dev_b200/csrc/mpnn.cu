@@ -51,7 +51,7 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kTrainTile = 64;                      // cells per tile of the training kernels
 // Pairs of a batch that go through the kernels together: as many as keep the
 // cells in flight at or below this (at least one pair) -- enough to fill the
-// GPU several times over, and a bounded workspace (about 1.9 KB per cell).
+// GPU several times over, and a bounded workspace (2.1 KB per cell, 540 MB).
 constexpr int64_t kTrainCells = 262144;
 
 }  // namespace mp

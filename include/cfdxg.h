@@ -182,7 +182,9 @@ int cfdxg_assemble_cell_diffusion(cfdxg_context* ctx, cfdxg_mesh* mesh,
  * HbyA, rAU: 3*n_cells SoA; p: n_cells; p_bc_fixed / p_bc_value: per patch.
  * If *A_inout is NULL a matrix is allocated (symbolic pattern built once),
  * otherwise only its values are refreshed.  b: n_cells.  phiHbyA (n_faces)
- * and grad_p (3*n_cells) are optional outputs (NULL to skip). */
+ * and grad_p (3*n_cells) are optional outputs (NULL to skip).  The first call
+ * on a mesh allocates device scratch that stays with it: 32 bytes per face, and
+ * 24 per cell when grad_p is skipped. */
 int cfdxg_assemble_pressure_correction(cfdxg_context* ctx, cfdxg_mesh* mesh,
                                        const double* HbyA, const double* rAU, const double* p,
                                        double rho, const int32_t* p_bc_fixed,
@@ -582,7 +584,11 @@ int cfdxg_mpnn_bind(cfdxg_context* ctx, cfdxg_mpnn* net, cfdxg_mesh* mesh, const
 /* y = N(r) for one residual (FP64 in/out). */
 int cfdxg_mpnn_apply(cfdxg_context* ctx, cfdxg_mpnn* net, const double* r, double* y, int32_t mem);
 /* One Adam step on a batch of (residual, error) pairs: loss = mean over pairs of
- * (e - N(r))^T A (e - N(r)) / (e^T A e).  r, e: batch * n_cells, row-major. */
+ * (e - N(r))^T A (e - N(r)) / (e^T A e).  r, e: batch * n_cells, row-major.
+ * The first training call on a network (this one or cfdxg_mpnn_loss_grad)
+ * allocates its device workspace, which stays with the network and grows with
+ * later batches: about 2.1 KB for every cell of the pairs taken together -- at
+ * most 64 pairs and 262,144 cells (540 MB), or one pair of a larger mesh. */
 int cfdxg_mpnn_train_step(cfdxg_context* ctx, cfdxg_mpnn* net, const double* r, const double* e,
                           int32_t batch, float learning_rate, int32_t mem, double* loss);
 /* Sets the V-cycle M the network is trained in front of (NULL: the network
