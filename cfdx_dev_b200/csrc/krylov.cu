@@ -1034,8 +1034,9 @@ constexpr int kHeldEntries = 8;
 // iterations, and a barrier whose target had wrapped let its blocks pass).
 // A relaunch costs some 50 us in half a second.
 constexpr int kRunIterations = 1 << 16;
-constexpr int kRunMostBlocks = 8192;
+constexpr int kRunMostBlocks = 2048;
 static_assert((2ull * kRunIterations + 1) * kRunMostBlocks < (1ull << 31), "the arrival counter wraps");
+static_assert(8 * kRunMostBlocks <= (kFused + 1) * kWideBlocks, "the blocks' partials fit the multi-dot's");
 
 // Sums v[0..NS) and takes the maximum of v[NS..NV) over the grid; every thread
 // gets the results.  Also a grid-wide barrier: what the block's threads wrote
